@@ -165,7 +165,7 @@ int plan_grids(pm_batch* b, int desired) {
         t.G.cell = q.cell;
         t.G.S = q.S;
         t.G.guess = b->guess;
-        t.r = b->inst[(size_t)i].radius;
+        t.E = gather_reach(t.G, b->inst[(size_t)i].radius);
         t.k = b->inst[(size_t)i].k;
         t.cls = gather_class(t.k);
     }

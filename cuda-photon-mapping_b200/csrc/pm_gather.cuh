@@ -25,6 +25,20 @@ struct GatherGrid {
 // 100M-photon 4K frame 1.5 measured 27.9 ms against 27.4 at 2.0)
 constexpr float GATHER_GUESS = 1.6f;
 
+// What a radius means on a grid, the same for all its queries.
+struct GatherReach {
+    float r;
+    float r2;                  // largest float s with sqrtf(s) <= r (-1 if none): a photon at squared
+                               // distance s lies within r exactly when s <= r2
+    float bscale;              // histogram bins / r2
+    float sc, inv_sc;          // sub-cell edge, its reciprocal
+    float pad;                 // boxes are taken this much larger
+    int rc;                    // half width in cells of the reference's cube, ceil(r / cell)
+                               // (CudaPhotonMapping/PhotonGrid.cu:257-284)
+    int sh;                    // log2 S
+};
+GatherReach gather_reach(const GatherGrid& G, float r);
+
 struct GatherQueries {
     int64_t n;
     // either packed 3-float arrays ...
@@ -61,7 +75,7 @@ cudaError_t gather(const GatherGrid& G, const GatherQueries& Q, float r, int k, 
 // ---- requests of several instances in one work queue ----
 struct GatherInstDev {
     GatherGrid G;
-    float r;
+    GatherReach E;            // gather_reach(G, r)
     int k;
     int cls;                  // gather_class(k): which store size answers it
 };
