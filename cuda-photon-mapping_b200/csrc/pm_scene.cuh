@@ -88,6 +88,25 @@ __device__ __forceinline__ bool model_gate(const float* c, V3 o, V3 d) {
     return tmin <= tmax;
 }
 
+// model_gate without its six divisions where the answer is clear: true only when
+// the gate passes.  With [a_i, b_i] the slab intervals along the axes (a_i <= b_i
+// whatever the rounding: rounded subtraction and division are monotone, and a
+// flat box has a_i == b_i), the gate passes when a_i <= b_j for all i != j and
+// b_j >= 0.  The intervals come from the slab terms ix = 1/d, ox = o ix as fused
+// multiply-adds; `e` is over four times their error.  NaN: false.
+__device__ __forceinline__ bool model_gate_clear(const float* c, float ix, float iy, float iz, float ox, float oy,
+                                                 float oz) {
+    const float x0 = __fmaf_rn(c[0], ix, -ox), x1 = __fmaf_rn(c[3], ix, -ox);
+    const float y0 = __fmaf_rn(c[1], iy, -oy), y1 = __fmaf_rn(c[4], iy, -oy);
+    const float z0 = __fmaf_rn(c[2], iz, -oz), z1 = __fmaf_rn(c[5], iz, -oz);
+    const float ex = 2e-6f * (fmax3(fabsf(x0), fabsf(x1), 0.f) + fabsf(ox));
+    const float ey = 2e-6f * (fmax3(fabsf(y0), fabsf(y1), 0.f) + fabsf(oy));
+    const float ez = 2e-6f * (fmax3(fabsf(z0), fabsf(z1), 0.f) + fabsf(oz));
+    const float ax = fminf(x0, x1) + ex, ay = fminf(y0, y1) + ey, az = fminf(z0, z1) + ez;
+    const float bx = fmaxf(x0, x1) - ex, by = fmaxf(y0, y1) - ey, bz = fmaxf(z0, z1) - ez;
+    return fmax3(ay, az, 0.f) <= bx && fmax3(ax, az, 0.f) <= by && fmax3(ax, ay, 0.f) <= bz;
+}
+
 __device__ __forceinline__ int hit_model_raw(const DevScene& S, int tri) {
     return __float_as_int(__ldg(&S.tri[5 * (size_t)tri + 2].w));
 }
@@ -285,7 +304,8 @@ __device__ __forceinline__ bool trav_step(const DevScene& S, Trav& T, V3 o, V3 d
                 const unsigned long long bit = 1ull << m;
                 if (!(T.gate_known & bit)) {
                     T.gate_known |= bit;
-                    if (model_gate(S.maabb + 6 * m, o, d)) T.gate_pass |= bit;
+                    if (model_gate_clear(S.maabb + 6 * m, ix, iy, iz, -nox, -noy, -noz) || model_gate(S.maabb + 6 * m, o, d))
+                        T.gate_pass |= bit;
                 }
                 pass = (T.gate_pass & bit) != 0ull;
             } else {
