@@ -261,8 +261,11 @@ int launch_stages(pm_batch* b, int stage, int* launches) {
         GatherQueries Q{};
         Q.n = b->req_cap; Q.pos4 = R.a; Q.nrm4 = R.b; Q.flag_mask = 1u;
         GatherOut O{P<float>(b->est_g), nullptr, nullptr, nullptr};
+        int max_k[2] = {0, 0};
+        for (const auto& I : b->inst) max_k[gather_class(I.k)] = std::max(max_k[gather_class(I.k)], I.k);
         BCK(gather_multi(P<GatherInstDev>(b->t_gather), P<int64_t>(b->t_px_off), b->n, Q, R.c, R.counter,
-                         b->req_split, P<unsigned long long>(b->queues), O, b->gather_warps, b->sm_count, b->st));
+                         b->req_split, P<unsigned long long>(b->queues), O, b->gather_warps, max_k,
+                         b->sm_count, b->st));
         L += (b->req_split > 0 ? 1 : 0) + (b->req_split < b->req_cap ? 1 : 0);
     }
     if (stage < 0 || stage == 4) {

@@ -14,8 +14,8 @@
 // One warp per query.  Photons are stored by (cell, sub-cell); the warp scans
 // the query's sub-cell and its 26 neighbours, then, with k candidates found,
 // the rest of the sub-cells that the bound on the k-th distance reaches, within
-// the reference's cube of cells.  With fewer than k it doubles the block of
-// sub-cells until k are found or the radius is covered.  Runs of photons with
+// the reference's cube of cells.  With fewer than k it scans the sphere that
+// should hold them, a larger one until it does or the radius is covered.  Runs of photons with
 // consecutive slots are queued and scanned as one list, one photon per lane
 // (one 16-byte load each); a photon whose squared distance is within the bound
 // goes to a per-warp shared-memory store (squared distance, slot) by ballot and
@@ -28,17 +28,21 @@
 // (z, y, x) order if those 27 hold k photons within r, else by shells of equal
 // Chebyshev distance (shell_index).
 //
-// What bounds it: instruction issue (0.78 of the issue slots; candidates come
-// from L1 / L2, 87 % L1 hits).  Against a store of 64-bit (distance, id) keys with
-// a root per candidate and the set-up by the whole warp: 2,340 -> 1,480 warp
-// instructions per query and 3.03 -> 2.23 ms for the 1.23M queries (k 64) of the
-// 10M-photon 1080p frame; k 128 on 2M photons 2.12 -> 1.53 ms, k 200 on 30M
-// photons 7.0 -> 6.1 ms, k 32 on 500K photons 2.03 -> 1.31 ms.  Loops are not
-// unrolled: the unrolled kernel waited for its instructions (2.6 of 10 stall
-// cycles per issue), 2.78 ms.
+// What bounds it: instruction issue (0.76 of the issue slots; candidates come
+// from L1 / L2).  Against a store of 64-bit (distance, id) keys with a root per
+// candidate, sub-cells tested one by one and the set-up by the whole warp: 2,340 ->
+// 1,330 warp instructions per query and 3.03 -> 1.92 ms for the 1.23M queries
+// (k 64) of the 10M-photon 1080p frame; k 128 on 2M photons 2.12 -> 1.27 ms,
+// k 200 on 30M photons 7.0 -> 5.4 ms, k 32 on 500K photons 2.03 -> 1.27 ms.
+// Loops are not unrolled and the scan is there once: with three unrolled copies
+// the kernel waited for its instructions (2.6 of 10 stall cycles per issue,
+// 2.78 ms).  A dense caustic (60,000 photons in 27 sub-cells) makes single
+// queries of 1 ms; a loop of its own for long runs made every other query 7 %
+// slower.
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <type_traits>
 #include "pm_gather.cuh"
 #include "pm_device.cuh"
 
@@ -70,7 +74,7 @@ struct Staged {
     float block2;             // squared distance to the nearest face of the 27 sub-cells with sub-cells behind it
     float bscale;             // NB / lim2
 };
-enum { Q_ACTIVE = 1, Q_GUESSED = 2 };
+enum { Q_ACTIVE = 1, Q_GUESSED = 2, Q_WIDE = 4 };
 
 // Shared memory of a block of NW warps: its queries and each warp's store.
 template <int UCAP, int NW>
@@ -107,34 +111,8 @@ __device__ __forceinline__ int small_div(int u, int d, float inv) {
     return q;
 }
 
-// Offsets of the t-th sub-cell of the shell at Chebyshev distance R around a
-// sub-cell (side = 2R + 1; 2 side^2 + 4 (side - 1)(side - 2) members): the two
-// full z faces, then the perimeter of each inner z layer.
-__device__ __forceinline__ void shell_member(int t, int R, int side, float inv_side, float inv_per, int& dx,
-                                             int& dy, int& dz) {
-    const int sq = side * side;
-    int x, y;
-    if (t < 2 * sq) {
-        const bool lo = t < sq;
-        dz = lo ? -R : R;
-        const int u = lo ? t : t - sq;
-        y = small_div(u, side, inv_side);
-        x = u - y * side;
-    } else {
-        const int e = side - 1, per = 4 * e;
-        const int u = t - 2 * sq;
-        const int layer = small_div(u, per, inv_per);
-        const int p = u - layer * per;
-        dz = -R + 1 + layer;
-        if (p < e) { x = p; y = 0; }
-        else if (p < 2 * e) { x = e; y = p - e; }
-        else if (p < 3 * e) { x = 3 * e - p; y = e; }
-        else { x = 0; y = 4 * e - p; }
-    }
-    dx = x - R;
-    dy = y - R;
-}
-// its inverse: t of the member at offset (dx, dy, dz)
+// Place of the sub-cell at offset (dx, dy, dz) in its shell at Chebyshev distance
+// R: the two full z faces (y, x order), then the perimeter of each inner z layer.
 __device__ __forceinline__ uint32_t shell_index(int dx, int dy, int dz, int R) {
     const int side = 2 * R + 1, e = side - 1, x = dx + R, y = dy + R;
     if (dz == -R) return (uint32_t)(y * side + x);
@@ -412,6 +390,11 @@ __device__ __forceinline__ void stage_query(const GatherGrid& G, const GatherRea
             s.lim2 = g2;
             flags |= Q_GUESSED;
         }
+    } else if (N < (uint32_t)k) {
+        // fewer than k in the block: the sphere of the guess, beyond the block
+        const float per = G.guess > 0.f ? G.guess : GATHER_GUESS;
+        s.lim2 = fminf(r2, N > 0u ? 9.f * sc * sc * (per * (float)k) / (3.14159265f * (float)N) : 64.f * sc * sc);
+        flags |= Q_WIDE;
     }
     auto face = [&](float p, float mn, int X, int lo, int hi) {
         const float a = X - 1 > lo ? p - (mn + (X - 1) * sc) : INFINITY, b = X + 1 < hi ? mn + (X + 2) * sc - p : INFINITY;
@@ -426,16 +409,6 @@ __device__ __forceinline__ void stage_query(const GatherGrid& G, const GatherRea
     s.bscale = (float)NB / s.lim2;
 }
 
-__device__ __forceinline__ int cube_size(const Cube& C) {
-    return (C.x1 - C.x0 + 1) * (C.y1 - C.y0 + 1) * (C.z1 - C.z0 + 1);
-}
-// the t-th cell of a cube of at most 1024, (z, y, x) order
-__device__ __forceinline__ uint32_t cube_cell(const GatherGrid& G, const Cube& C, int t) {
-    const int nx = C.x1 - C.x0 + 1, ny = C.y1 - C.y0 + 1;
-    const int row = small_div(t, nx, rcp((float)nx)), z = small_div(row, ny, rcp((float)ny));
-    return (uint32_t)(C.x0 + t - row * nx + (C.y0 + row - z * ny) * G.gx + (C.z0 + z) * G.gx * G.gy);
-}
-
 // Sub-cells [range_low, range_high] along an axis hold every photon within
 // reach of f (both in sub-cell units), clamped to [lo, hi].  Taken wide: a
 // sub-cell too many costs time only, its photons fail the distance test.
@@ -446,18 +419,109 @@ __device__ __forceinline__ int range_high(float f, float reach, int lo, int hi) 
     return (int)fminf(fmaxf(floorf(f + reach + fabsf(f) * 1e-6f), (float)lo), (float)hi);
 }
 
-// photons of a cube of cells that are scanned without looking at its sub-cells,
-// when the 27 around the query hold too few
-constexpr uint32_t SPARSE_MAX = 1024;
+// Ascending sort of keys[0, n), n <= 32 NR, one warp, NR keys per lane in
+// registers (bitonic).
+template <int NR>
+__device__ __noinline__ void sort_u32(uint32_t* keys, int n, int lane) {
+    uint32_t v[NR];
+#pragma unroll
+    for (int r = 0; r < NR; r++) v[r] = 32 * r + lane < n ? keys[32 * r + lane] : 0xffffffffu;
+#pragma unroll
+    for (int size = 2; size <= 32 * NR; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride >= 32; stride >>= 1)
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                const int o = r ^ (stride >> 5);
+                if (o > r) {
+                    const uint32_t lo = min(v[r], v[o]), hi = max(v[r], v[o]);
+                    const bool up = ((32 * r) & size) == 0;
+                    v[r] = up ? lo : hi;
+                    v[o] = up ? hi : lo;
+                }
+            }
+#pragma unroll 1
+        for (int stride = min(size >> 1, 16); stride > 0; stride >>= 1)
+#pragma unroll
+            for (int r = 0; r < NR; r++) {
+                const uint32_t o = __shfl_xor_sync(0xffffffffu, v[r], stride);
+                const bool up = ((32 * r + lane) & size) == 0, lower = (lane & stride) == 0;
+                v[r] = up == lower ? min(v[r], o) : max(v[r], o);
+            }
+    }
+#pragma unroll
+    for (int r = 0; r < NR; r++)
+        if (32 * r + lane < n) keys[32 * r + lane] = v[r];
+    __syncwarp();
+}
 
-// What a warp scans next: the query's sub-cell and its 26 neighbours; a shell
-// of sub-cells; all cells of the cube; the rows of sub-cells of a box.
-enum { M_RING = 0, M_SHELL = 1, M_CELLS = 2, M_BOX = 3 };
+// The store's cnt candidates, found block by block, into the shells' order: to
+// the store's upper half, by keys (sub-cell's place in the walk of shells, scan
+// order; cnt <= k <= UCAP / 2; inside a sub-cell the scan order is the slots').
+template <int UCAP>
+__device__ __forceinline__ void shells_order(const GatherGrid& G, const GatherReach& E, WarpStore<UCAP>& U, const Staged& s,
+                                          int cnt, int lane) {
+    __syncwarp();
+    uint2* out = U.ent + UCAP / 2;
+    unsigned long long* key = reinterpret_cast<unsigned long long*>(out);
+    uint32_t* key32 = reinterpret_cast<uint32_t*>(out);
+    // pass 0: 24-bit places (shells up to 127); pass 1, when one does not fit: 64-bit keys
+    int wide = 0;
+#pragma unroll 1
+    for (; wide < 2; wide++) {
+        bool fits = true;
+#pragma unroll 1
+        for (int e = lane; e < cnt; e += 32) {
+            const float4 p = __ldg(G.gpos + U.ent[e].y);
+            int cx, cy, cz, ux, uy, uz;
+            locate(p.x, G.mn[0], G.cell, G.gx, G.S, cx, ux);
+            locate(p.y, G.mn[1], G.cell, G.gy, G.S, cy, uy);
+            locate(p.z, G.mn[2], G.cell, G.gz, G.S, cz, uz);
+            const int dx = (cx << E.sh) + ux - s.X0, dy = (cy << E.sh) + uy - s.Y0, dz = (cz << E.sh) + uz - s.Z0;
+            const int R = max(max(abs(dx), abs(dy)), abs(dz));
+            const uint32_t t = R <= 1 ? (uint32_t)(9 * (dz + 1) + 3 * (dy + 1) + dx + 1) : shell_index(dx, dy, dz, R);
+            if (wide) {
+                key[e] = ((unsigned long long)(R <= 1 ? 0 : R) << 32 | t) << 10 | (unsigned long long)e;
+            } else {
+                const uint32_t inside = R <= 1 ? 0u : (uint32_t)((2 * R - 1) * (2 * R - 1) * (2 * R - 1));
+                key32[e] = (inside + t) << 8 | (uint32_t)e;
+                fits = fits && R <= 127;
+            }
+        }
+        __syncwarp();
+        if (wide) {
+            warp_sort_keys(key, cnt, lane);
+        } else if (__all_sync(0xffffffffu, fits)) {
+            if (cnt <= 64) sort_u32<2>(key32, cnt, lane);
+            else if (cnt <= 128) sort_u32<4>(key32, cnt, lane);
+            else sort_u32<8>(key32, cnt, lane);
+            break;
+        }
+    }
+    uint2 v[8];   // cnt <= 256
+#pragma unroll
+    for (int r = 0; r < 8; r++)
+        if (32 * r + lane < cnt)
+            v[r] = U.ent[wide ? (int)(key[32 * r + lane] & 1023ull) : (int)(key32[32 * r + lane] & 255u)];
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < 8; r++)
+        if (32 * r + lane < cnt) out[32 * r + lane] = v[r];
+    __syncwarp();
+}
+
+// What a warp scans: the query's sub-cell and its 26 neighbours; the rest of a
+// bound's sphere; or (too few in the 27) a whole sphere that grows until it holds
+// k or reaches r, by its sub-cells or, from 4 sub-cells on, by its cells unless
+// those hold more than COARSE_MAX photons.
+enum { M_RING = 0, M_REST = 1, M_WIDE = 2 };
+constexpr uint32_t COARSE_MAX = 1536;
 
 // one staged query (one warp): the k nearest photons within r and the estimate
-// (UNI: G.pow_uniform is honoured; the batch kernel, whose instance table is
-// copied per query, reads the power array instead and keeps its registers;
-// inv_norm: 1 / (1 - exp(-1.953)))
+// (UNI: G.pow_uniform is honoured; the batch kernel reads the power array
+// instead.  Its G and E are its instance's in global memory, read where they are
+// used: copied to registers per query, the 16-instance gather took 16.3 ms
+// instead of 13.7.  inv_norm: 1 / (1 - exp(-1.953)))
 template <int UCAP, bool UNI = true>
 __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherReach& E, WarpStore<UCAP>& U,
                                              const Staged& s, int64_t i, const float* __restrict__ pnrm, int k,
@@ -468,28 +532,55 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
     float bscale = s.bscale;   // histogram bin of d2 = min(NB - 1, (int)(d2 * bscale))
     uint32_t found = 0u;       // find_bin's answer for a store of `fn`
     int fn = -1;
-    bool guessed = (s.flags & Q_GUESSED) != 0;
-    bool sorted = true;        // the store is in the estimate's order
-    int mode = M_RING, base = 0, total = 27;
-    int h = 1, R = 2;          // half width of the block already scanned; the next shell or box
+    int mode = s.flags & Q_WIDE ? M_WIDE : M_RING, base = 0, total = 27;
+    bool coarse = false;       // M_WIDE: rows of cells, not of sub-cells
+    bool plan = mode == M_WIDE;   // the box of rows is still to be set
     const float m2 = 1.f + 2e-5f;
     reinterpret_cast<uint2*>(U.dh)[lane] = make_uint2(0u, 0u);
     __syncwarp();
+    coarse = plan && lim2 > 16.f * E.sc * E.sc && E.sh > 0;
 #pragma unroll 1
     while (true) {
-        // ---- up to 32 (box: 64) runs of photons, one or two per lane
+        const int sh = coarse ? 0 : E.sh;               // log2 of the units per cell
+        const float unit = coarse ? G.cell : E.sc;
+        if (plan) {
+            // The box, in units, that the sphere of squared radius lim2 can
+            // reach inside the cube.  One lane per (row of units along x, cell the
+            // row crosses): the sub-cells of a row inside one cell have
+            // consecutive keys, so their photons are one run of slots (two where
+            // the 27 sub-cells cut the row), and so have all cells of a row.
+            plan = false;
+            const float inv = coarse ? 1.f / G.cell : E.inv_sc;
+            const int X0 = s.X0 >> (E.sh - sh), Y0 = s.Y0 >> (E.sh - sh), Z0 = s.Z0 >> (E.sh - sh);
+            const Cube C = cube_of(G, E, X0 >> sh, Y0 >> sh, Z0 >> sh);
+            const float reach = (sqrt_approx(lim2 * m2) * (1.f + 1e-5f) + E.pad) * inv + 0.01f;
+            const float fx = (s.qx - G.mn[0]) * inv, fy = (s.qy - G.mn[1]) * inv, fz = (s.qz - G.mn[2]) * inv;
+            const int x0 = range_low(fx, reach, C.x0 << sh, X0), x1 = range_high(fx, reach, X0, ((C.x1 + 1) << sh) - 1);
+            const int y0 = range_low(fy, reach, C.y0 << sh, Y0), y1 = range_high(fy, reach, Y0, ((C.y1 + 1) << sh) - 1);
+            const int z0 = range_low(fz, reach, C.z0 << sh, Z0), z1 = range_high(fz, reach, Z0, ((C.z1 + 1) << sh) - 1);
+            if (mode == M_REST && x0 >= X0 - 1 && x1 <= X0 + 1 && y0 >= Y0 - 1 && y1 <= Y0 + 1 && z0 >= Z0 - 1 && z1 <= Z0 + 1)
+                break;
+            const int runs = sh == 0 ? 1 : (x1 >> sh) - (x0 >> sh) + 1;
+            const int ny = y1 - y0 + 1;
+            total = ny * (z1 - z0 + 1) * runs;
+            base = 0;
+            if (coarse && total > 64) {
+                coarse = false;
+                plan = true;
+                continue;
+            }
+            __syncwarp();
+            if (lane == 0) {
+                U.box[0] = x0; U.box[1] = x1; U.box[2] = y0; U.box[3] = ny; U.box[4] = z0; U.box[5] = runs;
+            }
+            __syncwarp();
+        }
+        // ---- up to 32 (M_REST: 64) runs of photons, one or two per lane
         uint32_t a = 0u, b = 0u, a2 = 0u, b2 = 0u;
         const int t = base + lane;
-        if (mode <= M_SHELL) {
-            int dx, dy, dz;
-            if (mode == M_RING) {
-                const int t3 = t / 3, t9 = t3 / 3;
-                dx = t - 3 * t3 - 1; dy = t3 - 3 * t9 - 1; dz = t9 - 1;
-            } else {
-                const int side = 2 * R + 1;
-                shell_member(min(t, total - 1), R, side, rcp((float)side), rcp((float)(4 * (side - 1))), dx, dy, dz);
-            }
-            const int X = s.X0 + dx, Y = s.Y0 + dy, Z = s.Z0 + dz, sh = E.sh;
+        if (mode == M_RING) {
+            const int t3 = t / 3, t9 = t3 / 3;
+            const int X = s.X0 + t - 3 * t3 - 1, Y = s.Y0 + t3 - 3 * t9 - 1, Z = s.Z0 + t9 - 1;
             const Cube C = cube_of(G, E, s.X0 >> sh, s.Y0 >> sh, s.Z0 >> sh);
             const int cx = X >> sh, cy = Y >> sh, cz = Z >> sh;
             if (t < total && cx >= C.x0 && cx <= C.x1 && cy >= C.y0 && cy <= C.y1 && cz >= C.z0 && cz <= C.z1) {
@@ -505,56 +596,48 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
                     b = __ldg(G.key_starts + key + 1);
                 }
             }
-        } else if (mode == M_BOX) {
-            // The sub-cells that the sphere of squared radius lim2 can reach
-            // in the block's box, minus the block |dx|, |dy|, |dz| <= h already
-            // scanned.  One lane per (row of sub-cells along x, cell the row
-            // crosses): the sub-cells of a row inside one cell have consecutive
-            // keys, so their photons are one run of slots (two where the
-            // scanned block cuts the row).  Rows in (z, y) order and runs in x
-            // order: the photons come in (z, y, x) order of their sub-cells.
+        } else {
+            // Rows in (z, y) order and runs in x order: the photons come in
+            // (z, y, x) order of their sub-cells (M_REST; M_WIDE sorts).
             const int x0 = U.box[0], x1 = U.box[1], y0 = U.box[2], ny = U.box[3], z0 = U.box[4], runs = U.box[5];
-            const int sh = E.sh, S = G.S;
             const int row = runs == 1 ? t : small_div(t, runs, rcp((float)runs)), run = t - row * runs;
             const int iz = small_div(row, ny, rcp((float)ny));
             const int Y = y0 + row - iz * ny, Z = z0 + iz;
-            const float gy = axis_gap(s.qy, G.mn[1] + Y * E.sc - E.pad, G.mn[1] + (Y + 1) * E.sc + E.pad, Y == 0,
+            const float gy = axis_gap(s.qy, G.mn[1] + Y * unit - E.pad, G.mn[1] + (Y + 1) * unit + E.pad, Y == 0,
                                       Y == (G.gy << sh) - 1);
-            const float gz = axis_gap(s.qz, G.mn[2] + Z * E.sc - E.pad, G.mn[2] + (Z + 1) * E.sc + E.pad, Z == 0,
+            const float gz = axis_gap(s.qz, G.mn[2] + Z * unit - E.pad, G.mn[2] + (Z + 1) * unit + E.pad, Z == 0,
                                       Z == (G.gz << sh) - 1);
             const float rem = lim2 * m2 - gy * gy - gz * gz;
             if (t < total && rem >= 0.f) {
-                const float fx = (s.qx - G.mn[0]) * E.inv_sc;
-                const float rx = (sqrt_approx(rem) * (1.f + 1e-5f) + E.pad) * E.inv_sc + 0.01f;
+                const float inv = coarse ? rcp(G.cell) : E.inv_sc;
+                const float fx = (s.qx - G.mn[0]) * inv;
+                const float rx = (sqrt_approx(rem) * (1.f + 1e-5f) + E.pad) * inv + 0.01f;
                 int xa = range_low(fx, rx, x0, x1), xb = range_high(fx, rx, x0, x1);
-                uint32_t kb;
-                if (S == 1) {
-                    kb = (uint32_t)((Y + Z * G.gy) * G.gx);
+                if (sh == 0) {
+                    const uint32_t* ks = G.key_starts + ((size_t)((Y + Z * G.gy) * G.gx + xa) << (3 * E.sh));
+                    a = __ldg(ks);
+                    b = __ldg(ks + ((size_t)(xb + 1 - xa) << (3 * E.sh)));
+                    if (mode == M_REST && abs(Y - s.Y0) <= 1 && abs(Z - s.Z0) <= 1) {   // (sub-cells: S = 1)
+                        b2 = b;
+                        b = __ldg(ks + (min(max(s.X0 - 1, xa), xb + 1) - xa));
+                        a2 = __ldg(ks + (min(max(s.X0 + 2, xa), xb + 1) - xa));
+                    }
                 } else {
                     const int c = (x0 >> sh) + run;
                     xa = max(xa, c << sh);
-                    xb = min(xb, (c << sh) + S - 1);
-                    kb = sub_key(G, c << sh, Y, Z, sh) - (uint32_t)(c << sh);
-                }
-                const int X0 = s.X0;
-                const bool inner = abs(Y - s.Y0) <= h && abs(Z - s.Z0) <= h;
-                const int left = inner ? min(xb, X0 - h - 1) : xb;
-                if (xa <= left) {
-                    a = __ldg(G.key_starts + (uint32_t)(kb + (uint32_t)xa));
-                    b = __ldg(G.key_starts + (uint32_t)(kb + (uint32_t)left + 1u));
-                }
-                const int right = max(xa, X0 + h + 1);
-                if (inner && right <= xb) {
-                    a2 = __ldg(G.key_starts + (uint32_t)(kb + (uint32_t)right));
-                    b2 = __ldg(G.key_starts + (uint32_t)(kb + (uint32_t)xb + 1u));
+                    xb = min(xb, ((c + 1) << sh) - 1);
+                    if (xa <= xb) {
+                        const uint32_t* ks = G.key_starts + sub_key(G, xa, Y, Z, sh);
+                        a = __ldg(ks);
+                        b = __ldg(ks + (xb + 1 - xa));
+                        if (mode == M_REST && abs(Y - s.Y0) <= 1 && abs(Z - s.Z0) <= 1) {
+                            b2 = b;
+                            b = __ldg(ks + (min(max(s.X0 - 1, xa), xb + 1) - xa));
+                            a2 = __ldg(ks + (min(max(s.X0 + 2, xa), xb + 1) - xa));
+                        }
+                    }
                 }
             }
-        } else if (t < total) {
-            const int sh = E.sh;
-            const Cube C = cube_of(G, E, s.X0 >> sh, s.Y0 >> sh, s.Z0 >> sh);
-            const uint32_t cell = cube_cell(G, C, t);
-            a = __ldg(G.key_starts + ((size_t)cell << (3 * sh)));
-            b = __ldg(G.key_starts + ((size_t)(cell + 1) << (3 * sh)));
         }
         base += 32;
         const bool end = base >= total;
@@ -566,15 +649,25 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
             qn += __popc(m1) + __popc(mb);
             __syncwarp();
         }
-        // ---- the photons of 32 queued runs as one list, one photon per lane:
-        // list entry o lies in the last run that starts at or before it (the
-        // runs that started before this round of 32 plus those that start in it
-        // at or before this lane; runs are not empty)
+        if (!end && (qn < 32 || coarse)) continue;
+        if (coarse) {   // at most 64 runs: too many photons in them?
+            uint32_t sum = 0u;
+            for (int e = lane; e < qn; e += 32) sum += min(U.qc[e], COARSE_MAX + 1u);
+            if (__reduce_add_sync(0xffffffffu, sum) > COARSE_MAX) {
+                coarse = false;
+                plan = true;
+                qn = 0;
+                continue;
+            }
+        }
+        // ---- the photons of 32 queued runs at a time as one list, one photon
+        // per lane: list entry o lies in the last run that starts at or before
+        // it (the runs that started before this round of 32 plus those that
+        // start in it at or before this lane; runs are not empty)
 #pragma unroll 1
-        while (qn >= 32 || (end && qn > 0)) {
-            const int cnt = min(qn, 32);
+        for (int q0 = 0; q0 < qn; q0 += 32) {
             uint32_t ra = 0u, c = 0u;
-            if (lane < cnt) { ra = U.qa[lane]; c = U.qc[lane]; }
+            if (q0 + lane < qn) { ra = U.qa[q0 + lane]; c = U.qc[q0 + lane]; }
             uint32_t incl = c;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -582,20 +675,11 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
                 if (lane >= o) incl += y;
             }
             const uint32_t photons = __shfl_sync(0xffffffffu, incl, 31);
-            const uint32_t excl = lane < cnt ? incl - c : 0xffffffffu;
+            const uint32_t excl = q0 + lane < qn ? incl - c : 0xffffffffu;
             const uint32_t delta = ra - excl;
             const V3 q = v3(s.qx, s.qy, s.qz);
-            int before = -1;
-#pragma unroll 1
-            for (uint32_t p0 = 0; p0 < photons; p0 += 32) {
-                const uint32_t starts = __reduce_or_sync(0xffffffffu, bit_or_zero(excl - p0));
-                const uint32_t o = min(p0 + lane, photons - 1);   // lanes past the end read the last photon, unused
-                const uint32_t j = __shfl_sync(0xffffffffu, delta, before + __popc(starts & lanemask_le())) + o;
-                before += __popc(starts);
-                const float4 p = __ldg(G.gpos + j);
-                const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-                const float d2 = dx * dx + dy * dy + dz * dz;
-                const bool ok = d2 <= lim2 && p0 + lane < photons;
+            auto enter = [&](float d2, uint32_t j) {   // the lanes whose photon is within lim2
+                const bool ok = d2 <= lim2;
                 const unsigned m = __ballot_sync(0xffffffffu, ok);
                 if (ok) {
                     U.ent[n + __popc(m & lanemask_lt())] = make_uint2(__float_as_uint(d2), j);
@@ -607,110 +691,56 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
                     n = k;
                     fn = -1;
                 }
+            };
+            int before = -1;
+#pragma unroll 1
+            for (uint32_t p0 = 0; p0 < photons; p0 += 32) {
+                const uint32_t starts = __reduce_or_sync(0xffffffffu, bit_or_zero(excl - p0));
+                const uint32_t o = min(p0 + lane, photons - 1);   // lanes past the end read the last photon, unused
+                const uint32_t j = __shfl_sync(0xffffffffu, delta, before + __popc(starts & lanemask_le())) + o;
+                before += __popc(starts);
+                const float4 p = __ldg(G.gpos + j);
+                const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+                const float d2 = dx * dx + dy * dy + dz * dz;
+                enter(p0 + lane < photons ? d2 : INFINITY, j);
             }
-            // the runs behind them move up (at most 63)
-            __syncwarp();
-            qn -= cnt;
-            if (qn == 0) break;
-            uint32_t na[2], nc[2];
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const bool in = 32 * u + lane < qn;
-                na[u] = in ? U.qa[32 * (u + 1) + lane] : 0u;
-                nc[u] = in ? U.qc[32 * (u + 1) + lane] : 0u;
-            }
-            __syncwarp();
-#pragma unroll
-            for (int u = 0; u < 2; u++)
-                if (32 * u + lane < qn) { U.qa[32 * u + lane] = na[u]; U.qc[32 * u + lane] = nc[u]; }
-            __syncwarp();
         }
+        qn = 0;
+        __syncwarp();
         if (!end) continue;
 
         // ---- what next
-        base = 0;
-        if (mode == M_CELLS) break;
-        const bool have = n >= k;
-        if (have) {
-            if (mode == M_BOX && R == 0) break;   // the last box
-            if (fn != n) { found = find_bin(U.dh, k, lane); fn = n; }
+        if (mode == M_REST) break;
+        plan = true;
+        if (n >= k) {
+            if (mode == M_WIDE) break;
+            found = find_bin(U.dh, k, lane);
+            fn = n;
             // the k-th lies in that bin: its upper edge (with a margin over the rounding of d2 * bscale) bounds it
             if (bscale < 1e30f) lim2 = fminf(lim2, __fdividef((float)((found & 255u) + 1u), bscale) * m2);
-            if (mode == M_RING && lim2 * m2 < s.block2) break;
-        } else if (mode == M_RING && guessed) {
-            guessed = false;
-            lim2 = E.r2; bscale = E.bscale; n = 0; fn = -1;
-            reinterpret_cast<uint2*>(U.dh)[lane] = make_uint2(0u, 0u);
-            __syncwarp();
+            if (lim2 * m2 < s.block2) break;
+            mode = M_REST;
             continue;
         }
-        const int sh = E.sh, X0 = s.X0, Y0 = s.Y0, Z0 = s.Z0;
-        const Cube C = cube_of(G, E, X0 >> sh, Y0 >> sh, Z0 >> sh);
-        const int lx = C.x0 << sh, ly = C.y0 << sh, lz = C.z0 << sh;
-        const int hx = ((C.x1 + 1) << sh) - 1, hy = ((C.y1 + 1) << sh) - 1, hz = ((C.z1 + 1) << sh) - 1;
-        const int Rmax = max(max(max(X0 - lx, hx - X0), max(Y0 - ly, hy - Y0)), max(Z0 - lz, hz - Z0));
-        if (mode == M_RING && !have) {
-            if (Rmax <= 1) break;
-            // too few in the block: all photons of the cube if they are few
-            const int cells = cube_size(C);
-            if (cells <= 1024) {
-                uint32_t sum = 0u;
-#pragma unroll 1
-                for (int c = lane; c < cells; c += 32) {
-                    const uint32_t cell = cube_cell(G, C, c);
-                    sum += min(__ldg(G.key_starts + ((size_t)(cell + 1) << (3 * sh))) -
-                                   __ldg(G.key_starts + ((size_t)cell << (3 * sh))), SPARSE_MAX + 1u);
-                }
-                if (__reduce_add_sync(0xffffffffu, sum) <= SPARSE_MAX) {
-                    n = 0; fn = -1;
-                    reinterpret_cast<uint2*>(U.dh)[lane] = make_uint2(0u, 0u);
-                    __syncwarp();
-                    sorted = false;
-                    mode = M_CELLS;
-                    total = cells;
-                    continue;
-                }
-            }
-            mode = M_SHELL;
-            R = 1;
+        if (lim2 == E.r2) {           // all within r is found ...
+            if (mode == M_WIDE || s.block2 == INFINITY) break;
+            mode = M_WIDE;            // ... in the 27 sub-cells: with the guess that they give, or r
+            lim2 = fminf(E.r2, 9.f * E.sc * E.sc * GATHER_GUESS * __fdividef((float)k, 3.14159265f * (float)max(n, 1)));
+        } else if (mode == M_WIDE) {  // the sphere held too few: a larger one
+            lim2 = fminf(E.r2, lim2 * fmaxf(2.f, 1.5f * GATHER_GUESS * __fdividef((float)k, (float)max(n, 1))));
+        } else {                      // the guess held too few of the 27: all of theirs within r
+            lim2 = E.r2;
+            plan = false;
         }
-        if (mode == M_SHELL) {   // shells while the second finds the k, each nearest first
-            h = R;
-            if (R < Rmax && (have || R == 1)) {
-                if ((float)R * E.sc - E.pad > sqrt_approx(lim2) * (1.f + 1e-5f)) break;
-                R++;
-                const int side = 2 * R + 1;
-                total = 2 * side * side + 4 * (side - 1) * (side - 2);
-                continue;
-            }
-            if (have) break;
-        }
-        // boxes of twice the half width until k are found, then the box of the bound's sphere
-        if (mode == M_BOX) h = R;
-        if (h >= Rmax || (!have && (float)h * E.sc - E.pad > E.r * (1.f + 1e-5f))) break;
-        if (mode == M_SHELL) sorted = false;
-        const int hm = have ? Rmax : min(2 * h, Rmax);
-        mode = M_BOX;
-        R = have ? 0 : hm;
-        const float reach = (sqrt_approx(lim2 * m2) * (1.f + 1e-5f) + E.pad) * E.inv_sc + 0.01f;
-        const float fx = (s.qx - G.mn[0]) * E.inv_sc, fy = (s.qy - G.mn[1]) * E.inv_sc, fz = (s.qz - G.mn[2]) * E.inv_sc;
-        const int x0 = range_low(fx, reach, max(lx, X0 - hm), min(hx, X0 + hm));
-        const int x1 = range_high(fx, reach, max(lx, X0 - hm), min(hx, X0 + hm));
-        const int y0 = range_low(fy, reach, max(ly, Y0 - hm), min(hy, Y0 + hm));
-        const int y1 = range_high(fy, reach, max(ly, Y0 - hm), min(hy, Y0 + hm));
-        const int z0 = range_low(fz, reach, max(lz, Z0 - hm), min(hz, Z0 + hm));
-        const int z1 = range_high(fz, reach, max(lz, Z0 - hm), min(hz, Z0 + hm));
-        // nothing outside the block (then r is covered: a bound's box, or a sphere of r inside the block)
-        if (x0 >= X0 - h && x1 <= X0 + h && y0 >= Y0 - h && y1 <= Y0 + h && z0 >= Z0 - h && z1 <= Z0 + h) break;
-        const int runs = E.sh == 0 ? 1 : (x1 >> sh) - (x0 >> sh) + 1;   // at S = 1 the cells of a row have consecutive keys
-        const int ny = y1 - y0 + 1;
-        total = ny * (z1 - z0 + 1) * runs;
-        __syncwarp();
-        if (lane == 0) {
-            U.box[0] = x0; U.box[1] = x1; U.box[2] = y0; U.box[3] = ny; U.box[4] = z0; U.box[5] = runs;
-        }
+        coarse = plan && lim2 > 16.f * E.sc * E.sc && E.sh > 0;
+        bscale = lim2 == E.r2 ? E.bscale : __fdividef((float)NB, lim2);
+        n = 0;
+        fn = -1;
+        base = 0;
+        reinterpret_cast<uint2*>(U.dh)[lane] = make_uint2(0u, 0u);
         __syncwarp();
     }
+    const bool sorted = mode != M_WIDE;   // the store is in the estimate's order
 
     float smax;   // the largest squared distance of the answer
     if (n > k) {
@@ -727,29 +757,8 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
     const float rk = sqrtf(smax);
     uint2* ent = U.ent;
     if (!sorted && cnt > 0) {
-        // the candidates were found block by block: into the shells' order, by
-        // keys (shell, place in it, scan order) in the store's upper half (cnt
-        // <= k <= UCAP / 2; inside a sub-cell the scan order is the slots')
+        shells_order<UCAP>(G, E, U, s, cnt, lane);
         ent += UCAP / 2;
-        unsigned long long* key = reinterpret_cast<unsigned long long*>(ent);
-#pragma unroll 1
-        for (int e = lane; e < cnt; e += 32) {
-            const float4 p = __ldg(G.gpos + U.ent[e].y);
-            const int S = G.S, X0 = s.X0, Y0 = s.Y0, Z0 = s.Z0;
-            int cx, cy, cz, ux, uy, uz;
-            locate(p.x, G.mn[0], G.cell, G.gx, S, cx, ux);
-            locate(p.y, G.mn[1], G.cell, G.gy, S, cy, uy);
-            locate(p.z, G.mn[2], G.cell, G.gz, S, cz, uz);
-            const int dx = cx * S + ux - X0, dy = cy * S + uy - Y0, dz = cz * S + uz - Z0;
-            const int R = max(max(abs(dx), abs(dy)), abs(dz));
-            const unsigned long long order = R <= 1 ? (unsigned long long)(9 * (dz + 1) + 3 * (dy + 1) + dx + 1)
-                                                    : (unsigned long long)R << 32 | shell_index(dx, dy, dz, R);
-            key[e] = order << 10 | (unsigned long long)e;
-        }
-        __syncwarp();
-        warp_sort_keys(key, cnt, lane);
-#pragma unroll 1
-        for (int e = lane; e < cnt; e += 32) ent[e] = U.ent[(int)(key[e] & 1023ull)];
     }
     __syncwarp();
 
@@ -908,11 +917,13 @@ k_gather(GatherGrid G, GatherReach E, GatherQueries Q, int k, int require_full, 
                        (int)min((int64_t)per, Q.n - q0), k, require_full, O, filter_norm());
 }
 
-// queries a block takes at a time from n, for `blocks` resident ones: one per
-// thread, fewer (down to one per warp) where the blocks would not get several turns
+// Queries a block takes at a time from n, for `blocks` resident ones: one per
+// thread, fewer where the blocks would not get 16 turns (the last ones end
+// together; 4 turns: 0.07 ms more at 547K queries), but two per warp while
+// there are enough (the set-up of one alone costs a ninth at 62K queries).
 __host__ __device__ __forceinline__ int block_chunk(int64_t n, int64_t blocks, int warps) {
-    const int64_t c = n / (4 * blocks) / warps * warps;
-    return (int)(c < warps ? warps : c > 32 * warps ? 32 * warps : c);
+    const int64_t c = n / (16 * blocks) / warps * warps, least = n >= 4 * blocks * warps ? 2 * warps : warps;
+    return (int)(c < least ? least : c > 32 * warps ? 32 * warps : c);
 }
 
 // Listed queries, persistent: blocks take list positions from *queue until
@@ -1010,9 +1021,7 @@ k_gather_multi(const GatherInstDev* __restrict__ tab, const int64_t* __restrict_
                 if (flags < 0) return;
                 if (flags & Q_ACTIVE) {
                     const GatherInstDev& T = tab[flags >> 8];
-                    const GatherGrid G = T.G;
-                    const GatherReach E = T.E;
-                    gather_query<UCAP, false>(G, E, U, M.q[t], q0 + t, normal_of(Q, q0 + t), T.k, 0, O, inv_norm, lane);
+                    gather_query<UCAP, false>(T.G, T.E, U, M.q[t], q0 + t, normal_of(Q, q0 + t), T.k, 0, O, inv_norm, lane);
                 } else {
                     gather_zero(q0 + t, 0, O, lane);
                 }
@@ -1051,7 +1060,8 @@ cudaError_t launch_multi(const GatherInstDev* tab, const int64_t* px_off, int ni
 
 cudaError_t gather_multi(const GatherInstDev* tab, const int64_t* px_off, int ninst, const GatherQueries& Q,
                          const float4* rec_c, const unsigned long long* n_req, int64_t split,
-                         unsigned long long* queues, const GatherOut& O, int warps, int sm_count, cudaStream_t st) {
+                         unsigned long long* queues, const GatherOut& O, int warps, const int max_k[2], int sm_count,
+                         cudaStream_t st) {
     if (Q.n <= 0) return cudaSuccess;
     if (split < 0 || split > Q.n || O.ids || O.cnt || O.rk || Q.idx) return cudaErrorInvalidValue;
     cudaError_t e = cudaMemsetAsync(queues, 0, 16, st);
@@ -1065,17 +1075,20 @@ cudaError_t gather_multi(const GatherInstDev* tab, const int64_t* px_off, int ni
     GatherOut O1 = O;
     O1.rad = O.rad + 3 * split;
     const float4* c1 = rec_c + split;
-    if (warps == 4) {
-        if (Q0.n > 0 &&
-            (e = launch_multi<256, 4>(tab, px_off, ninst, Q0, rec_c, n_req, queues, 0, O, sm_count, st)) != cudaSuccess)
-            return e;
-        if (Q1.n > 0) e = launch_multi<512, 4>(tab, px_off, ninst, Q1, c1, n_req + 1, queues + 1, 1, O1, sm_count, st);
-        return e;
+    auto one = [&](auto ucap, const GatherQueries& q, const float4* c, int cls, const GatherOut& o) {
+        constexpr int U = decltype(ucap)::value;
+        return warps == 4 ? launch_multi<U, 4>(tab, px_off, ninst, q, c, n_req + cls, queues + cls, cls, o, sm_count, st)
+                          : launch_multi<U, 8>(tab, px_off, ninst, q, c, n_req + cls, queues + cls, cls, o, sm_count, st);
+    };
+    using std::integral_constant;
+    if (Q0.n > 0) {
+        e = max_k[0] <= 64 ? one(integral_constant<int, 192>(), Q0, rec_c, 0, O)
+                           : one(integral_constant<int, 256>(), Q0, rec_c, 0, O);
+        if (e != cudaSuccess) return e;
     }
-    if (Q0.n > 0 &&
-        (e = launch_multi<256, 8>(tab, px_off, ninst, Q0, rec_c, n_req, queues, 0, O, sm_count, st)) != cudaSuccess)
-        return e;
-    if (Q1.n > 0) e = launch_multi<512, 8>(tab, px_off, ninst, Q1, c1, n_req + 1, queues + 1, 1, O1, sm_count, st);
+    if (Q1.n > 0)
+        e = max_k[1] <= 160 ? one(integral_constant<int, 352>(), Q1, c1, 1, O1)
+                            : one(integral_constant<int, 512>(), Q1, c1, 1, O1);
     return e;
 }
 
