@@ -273,6 +273,26 @@ Layout layout(int n) {
     return L;
 }
 
+// Triangle records (pm_scene.cuh) with the operations of the reference's triangle
+// test (CudaPhotonMapping/Model.cuh:69-120); bound by its 36 + 80 bytes per triangle.
+__global__ void k_tri_records(const float* __restrict__ tri_pos, const int* __restrict__ tri_model, int n,
+                              float4* __restrict__ out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const float* p = tri_pos + 9 * (size_t)t;
+    const V3 v0 = ld3(p), v2 = ld3(p + 6);
+    const V3 e1 = vsub(ld3(p + 3), v0), e2 = vsub(v2, v0);
+    const V3 nn = vcross(e1, e2);
+    const float denom = 1.0f / vdot(nn, nn), nd0 = vdot(nn, v0);
+    const V3 f = vsub(v0, v2);
+    float4* r = out + 5 * (size_t)t;
+    r[0] = make_float4(v0.x, v0.y, v0.z, nd0);
+    r[1] = make_float4(e1.x, e1.y, e1.z, denom);
+    r[2] = make_float4(v2.x, v2.y, v2.z, __int_as_float(tri_model[t]));
+    r[3] = make_float4(f.x, f.y, f.z, 0.f);
+    r[4] = make_float4(nn.x, nn.y, nn.z, 0.f);
+}
+
 __global__ void k_leaf_records(const float4* __restrict__ tri, const int* __restrict__ prim, int n,
                                float4* __restrict__ out) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -287,6 +307,12 @@ __global__ void k_leaf_records(const float4* __restrict__ tri, const int* __rest
 }
 
 }  // namespace
+
+cudaError_t tri_records(const float* tri_pos, const int* tri_model, int ntri, float4* out, cudaStream_t st) {
+    if (ntri <= 0) return cudaSuccess;
+    k_tri_records<<<blocks_of(ntri, 256), 256, 0, st>>>(tri_pos, tri_model, ntri, out);
+    return cudaGetLastError();
+}
 
 cudaError_t bvh_leaf_records(const float4* tri, const int* prim, int ntri, float4* out, cudaStream_t st) {
     if (ntri <= 0) return cudaSuccess;

@@ -19,6 +19,10 @@ inline int64_t lbvh_node_count(int ntri) { return ntri > 1 ? (int64_t)ntri - 1 :
 cudaError_t lbvh_build(const float* tri_pos, int ntri, float pad, float4* nodes, int* prim, void* scratch,
                        unsigned* status, int* launches, cudaStream_t st);
 
+// The 5-float4 triangle records of pm_scene.cuh (device arrays: 9 floats and one
+// model index per triangle).
+cudaError_t tri_records(const float* tri_pos, const int* tri_model, int ntri, float4* out, cudaStream_t st);
+
 // Triangle records in leaf order, 4 float4 each: out[j] = the first three
 // float4 of tri[prim[j]] and its fifth (the normal) with the triangle's index
 // in w (the fourth, v0 - v2, is formed by the test).
