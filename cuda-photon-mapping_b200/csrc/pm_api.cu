@@ -68,7 +68,7 @@ std::vector<DevBuf*> all_buffers(pm_ctx* ctx) {
                               &ctx->cache_loss, &ctx->est_mlp, &ctx->est_fb, &ctx->probe_pos, &ctx->probe_nrm,
                               &ctx->probe_req, &ctx->probe_est, &ctx->tile_flag, &ctx->learned_counts,
                               &ctx->fallback_list, &ctx->bvh_scratch, &ctx->tri_leaf, &ctx->eye_order, &ctx->rq_keys,
-                              &ctx->rq_k0, &ctx->rq_k1, &ctx->rq_v0, &ctx->rq_v1, &ctx->rq_hist, &ctx->rq_ws,
+                              &ctx->rq_k0, &ctx->rq_k1, &ctx->rq_v0, &ctx->rq_v1, &ctx->rq_hist,
                               &ctx->work, &ctx->eye_band};
     for (auto& m : ctx->maps)
         for (DevBuf* b : {&m.pos, &m.dir, &m.pow, &m.starts, &m.sizes, &m.gpos, &m.gdir, &m.gpow, &m.cid, &m.keys0,
@@ -1365,10 +1365,9 @@ int request_order(pm_ctx* ctx, FrameSetup& F, cudaStream_t st) {
     ENSURE(ctx->rq_k0, (size_t)n * 4); ENSURE(ctx->rq_k1, (size_t)n * 4);
     ENSURE(ctx->rq_v0, (size_t)n * 4); ENSURE(ctx->rq_v1, (size_t)n * 4);
     ENSURE(ctx->rq_hist, radix_hist_elems(n) * 4);
-    ENSURE(ctx->rq_ws, scan_workspace_bytes((int64_t)radix_hist_elems(n)));
     CK(request_keys(F.R.a, n, ctx->aabb, P<uint32_t>(ctx->rq_keys), st));
     RadixBuffers RB{{P<uint32_t>(ctx->rq_k0), P<uint32_t>(ctx->rq_k1)}, {P<uint32_t>(ctx->rq_v0), P<uint32_t>(ctx->rq_v1)},
-                    P<uint32_t>(ctx->rq_hist), ctx->rq_ws.p, P<unsigned>(ctx->status)};
+                    P<uint32_t>(ctx->rq_hist), P<unsigned>(ctx->status)};
     int launches = 0;
     CK(radix_sort_u32(RB, P<uint32_t>(ctx->rq_keys), nullptr, n, REQUEST_KEY_BITS, false, nullptr, &F.order, &launches,
                       st));

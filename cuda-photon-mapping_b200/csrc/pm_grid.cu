@@ -16,9 +16,11 @@
 //   scan_u32       exclusive scan of key counts (decoupled look-back) ->
 //                  key_starts; cell_starts / cell_sizes follow exactly
 //   LSD radix sort of the keys, <= 9 bits per pass, carrying the photon index:
-//     k_radix_upsweep    per-tile digit histogram, digit-major
-//     scan_u32           offsets of every (digit, tile)
-//     k_radix_downsweep  stable in-tile ranks (per-bit ballots) + scatter
+//     k_radix_count    digit counts of every block's run of keys
+//     k_radix_offsets  their prefixes over the blocks
+//     k_radix_pass     stable in-tile ranks (per-bit ballots) + scatter
+//     (up to 1.8M keys: k_radix_hist once, then k_radix_pass alone, its tiles
+//     looking back over each other)
 //   k_grid_gather  sorted photon index -> (pos, id), dir, power in slot order
 #include <cmath>
 #include <algorithm>
@@ -30,17 +32,21 @@ namespace pm {
 
 namespace {
 
-// 512 threads of 8 keys per tile (3 blocks, 48 warps per SM): grid build
-// 1.10 -> 1.03 ms per 10M photons against 256 x 16 (4 blocks, 32 warps) and
-// 256 x 8 (5 or 6 blocks, 1.07 ms); the ranking and staging phases are
-// latency bound, so more resident warps per SM pay.  RADIX_THREADS <=
-// RADIX_MAX_BINS (each thread owns whole bins in the downsweep's prefix).
+// 512 threads of 8 keys per tile (3 blocks, 48 warps per SM): the ranking and
+// staging phases are latency bound, so resident warps pay (256 x 16 keys, 32
+// warps: 7 % more for the grid build of 10M photons; 256 x 8: 4 %).
+// RADIX_THREADS >= RADIX_MAX_BINS (one thread per digit).
 constexpr int RADIX_THREADS = 512;
 constexpr int RADIX_ITEMS = 8;
 constexpr int RADIX_TILE = RADIX_THREADS * RADIX_ITEMS;
 constexpr int RADIX_WARPS = RADIX_THREADS / 32;
 constexpr int RADIX_MAX_BITS = 9;
 constexpr int RADIX_MAX_BINS = 1 << RADIX_MAX_BITS;
+static_assert(RADIX_THREADS >= RADIX_MAX_BINS, "one thread per digit");
+constexpr int RADIX_MAX_PASSES = 4;    // 32-bit keys, <= 9 bits each
+// Blocks of a pass, all resident (3 per SM by shared memory): up to as many tiles
+// one tile each, beyond that each block takes a run of consecutive tiles.
+constexpr int RADIX_BLOCKS = 3 * 148;
 
 struct GridGeom {
     float mnx, mny, mnz;
@@ -225,25 +231,60 @@ __global__ void k_cells_from_keys(const uint32_t* __restrict__ key_starts, int64
     sizes[c] = b - a;
 }
 
+// Digit histograms of all passes in one read of the keys: hist[p][digit].
 __global__ void __launch_bounds__(RADIX_THREADS)
-k_radix_upsweep(const uint32_t* __restrict__ keys, int64_t n, int shift, int bits, uint32_t* __restrict__ hist,
-                int tiles) {
-    __shared__ uint32_t h[RADIX_MAX_BINS];
-    const int tid = threadIdx.x, bins = 1 << bits;
-    const uint32_t dm = (uint32_t)bins - 1u;
-    for (int b = tid; b < bins; b += RADIX_THREADS) h[b] = 0;
+k_radix_hist(const uint32_t* __restrict__ keys, int64_t n, int width, int passes, uint32_t* __restrict__ hist) {
+    __shared__ uint32_t h[RADIX_MAX_PASSES][RADIX_MAX_BINS];
+    const int tid = threadIdx.x, bins = 1 << width;
+    for (int i = tid; i < RADIX_MAX_PASSES * RADIX_MAX_BINS; i += RADIX_THREADS) (&h[0][0])[i] = 0u;
     __syncthreads();
-    const int64_t base = (int64_t)blockIdx.x * RADIX_TILE;
-#pragma unroll 4
-    for (int i = 0; i < RADIX_ITEMS; i++) {
-        int64_t gi = base + i * RADIX_THREADS + tid;
-        if (gi < n) atomicAdd(&h[(keys[gi] >> shift) & dm], 1u);
+    const int64_t stride = (int64_t)gridDim.x * RADIX_THREADS;
+    for (int64_t i = (int64_t)blockIdx.x * RADIX_THREADS + tid; i < n; i += stride) {
+        const uint32_t k = keys[i];
+        for (int p = 0; p < passes; p++) atomicAdd(&h[p][(k >> (width * p)) & (uint32_t)(bins - 1)], 1u);
     }
     __syncthreads();
-    for (int b = tid; b < bins; b += RADIX_THREADS) hist[(int64_t)b * tiles + blockIdx.x] = h[b];
+    for (int p = 0; p < passes; p++)
+        for (int b = tid; b < bins; b += RADIX_THREADS)
+            if (h[p][b]) atomicAdd(hist + p * RADIX_MAX_BINS + b, h[p][b]);
 }
 
-// Stable scatter of one radix pass.  A warp owns 256 consecutive keys and walks
+// exclusive scan over the block's RADIX_THREADS values
+__device__ __forceinline__ uint32_t radix_block_scan(uint32_t v, uint32_t* wsum) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    uint32_t off = incl - v;
+    for (int w = 0; w < warp; w++) off += wsum[w];
+    return off;
+}
+
+// One radix pass: a stable scatter by one digit.
+//
+// Few keys (one tile per block, all blocks resident): the tiles find their
+// places themselves (one-sweep radix sort: Adinets & Merrill, "Onesweep", 2022,
+// over the decoupled look-back of Merrill & Garland, 2016).  Tiles take dynamic
+// ids; each publishes its count of every digit in one word (state, count), later
+// the count of it and all tiles before, and one thread per digit adds the words of
+// the tiles before its own up to the first of the second kind, four at a time.
+// The words of pass p have states 2p + 1 and 2p + 2, so those of earlier passes
+// read as not yet there and the array is cleared once per sort.  Every wait is
+// bounded (ST_TIMEOUT; the tile then writes nothing).
+// Many keys: each block scatters a run of consecutive tiles, whose digits' places
+// k_radix_count and k_radix_offsets have found.
+//
+// Bound by the latency of the in-tile ranking (0.5 of the issue slots).  Against
+// a histogram per tile, a scan over all (digit, tile) and a scatter of single
+// tiles: a pass over 10M keys 0.17 -> 0.13 ms (grid build 1.00 -> 0.96), grid build
+// of 100K photons 0.108 -> 0.096 ms, of 100M 14.8 -> 14.0.
+//
+// A warp owns 256 consecutive keys and walks
 // them 32 at a time in order; equal digits inside a step are ranked by lane
 // (the lanes of a digit found by one ballot per digit bit: grid build 1.14 ->
 // 1.10 ms against __match_any_sync), across steps by a per-warp running
@@ -257,113 +298,186 @@ struct RadixSmem {
     uint32_t dbase[RADIX_MAX_BINS];             // global start of the tile's run of each digit
     uint32_t lbase[RADIX_MAX_BINS];             // start of each digit inside the staged tile
     uint32_t wsum[RADIX_WARPS];
+    int tile, failed;
     uint32_t key[RADIX_TILE];
     uint32_t val[RADIX_TILE];
 };
 
+// the look-back's words: a state in the top 4 bits, a count below
+constexpr int WORD_SHIFT = 28;
+static_assert((int64_t)RADIX_BLOCKS * RADIX_TILE < ((int64_t)1 << WORD_SHIFT), "a count fits");
+
+// Digit counts of every block's run of keys, counts[block][digit].
+__global__ void __launch_bounds__(RADIX_THREADS)
+k_radix_count(const uint32_t* __restrict__ keys, int64_t n, int64_t run, int shift, int bins, uint32_t* __restrict__ counts) {
+    __shared__ uint32_t h[RADIX_MAX_BINS];
+    const int tid = threadIdx.x;
+    for (int b = tid; b < bins; b += RADIX_THREADS) h[b] = 0u;
+    __syncthreads();
+    const int64_t first = (int64_t)blockIdx.x * run, last = min(first + run, n);
+#pragma unroll 4
+    for (int64_t i = first + tid; i < last; i += RADIX_THREADS) atomicAdd(&h[(keys[i] >> shift) & (uint32_t)(bins - 1)], 1u);
+    __syncthreads();
+    for (int b = tid; b < bins; b += RADIX_THREADS) counts[(int64_t)blockIdx.x * bins + b] = h[b];
+}
+
+// One block per digit: counts[.][digit] becomes its exclusive prefix over the
+// blocks, totals[digit] its sum.
+__global__ void __launch_bounds__(RADIX_THREADS)
+k_radix_offsets(uint32_t* __restrict__ counts, int blocks, int bins, uint32_t* __restrict__ totals) {
+    __shared__ uint32_t wsum[RADIX_WARPS];
+    static_assert(RADIX_BLOCKS <= RADIX_THREADS, "one block of counts per thread");
+    uint32_t* c = counts + (int64_t)threadIdx.x * bins + blockIdx.x;
+    const bool in = (int)threadIdx.x < blocks;
+    const uint32_t v = in ? *c : 0u;
+    const uint32_t e = radix_block_scan(v, wsum);
+    if (in) *c = e;
+    if ((int)threadIdx.x == blocks - 1) totals[blockIdx.x] = e + v;
+}
+
+// RUNS: block i scatters the run of keys [i * run, ...) tile by tile, counts[i]
+// its digits' prefixes over the blocks, hist the digits' totals.  Else one tile,
+// whose digits' prefixes come from the look-back.
+template <bool RUNS>
 __global__ void __launch_bounds__(RADIX_THREADS, 3)   // 3 blocks per SM: the shared-memory limit
-k_radix_downsweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, int64_t n, int shift,
-                  int bits, const uint32_t* __restrict__ offsets, int tiles, uint32_t* __restrict__ keys_out,
-                  uint32_t* __restrict__ vals_out) {
+k_radix_pass(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in, int64_t n, int64_t run, int width,
+             int pass, const uint32_t* __restrict__ hist, uint32_t* __restrict__ words, unsigned* __restrict__ tile_counter,
+             uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, unsigned* status) {
     extern __shared__ __align__(16) unsigned char radix_smem[];
     RadixSmem& R = *reinterpret_cast<RadixSmem*>(radix_smem);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, bins = 1 << bits;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, bins = 1 << width, shift = width * pass, bits = width;
     const uint32_t dm = (uint32_t)bins - 1u;
-    for (int i = tid; i < RADIX_WARPS * RADIX_MAX_BINS; i += RADIX_THREADS) (&R.wh[0][0])[i] = 0u;
-    for (int b = tid; b < bins; b += RADIX_THREADS) R.dbase[b] = offsets[(int64_t)b * tiles + blockIdx.x];
-    __syncthreads();
-    const int64_t tbase = (int64_t)blockIdx.x * RADIX_TILE;
-    const int64_t wbase = tbase + (int64_t)warp * (32 * RADIX_ITEMS);
-    const int tcount = (int)min((int64_t)RADIX_TILE, n - tbase);
-    uint32_t k[RADIX_ITEMS], v[RADIX_ITEMS], r[RADIX_ITEMS];
-#pragma unroll
-    for (int j = 0; j < RADIX_ITEMS; j++) {
-        int64_t gi = wbase + j * 32 + lane;
-        bool valid = gi < n;
-        unsigned vm = __ballot_sync(0xffffffffu, valid);
-        k[j] = valid ? keys_in[gi] : 0u;
-        v[j] = valid ? (vals_in ? vals_in[gi] : (uint32_t)gi) : 0u;
-        r[j] = 0u;
-        // lanes holding the same digit: one ballot per digit bit (independent
-        // instructions, where a match has one long latency)
-        const uint32_t d = (k[j] >> shift) & dm;
-        unsigned peers = vm;
-#pragma unroll
-        for (int b = 0; b < RADIX_MAX_BITS; b++) {
-            if (b < bits) {
-                const unsigned on = __ballot_sync(0xffffffffu, (d >> b) & 1u);
-                peers &= ((d >> b) & 1u) ? on : ~on;
-            }
+    const unsigned part = 2u * pass + 1u, whole = part + 1u;
+    const int b = tid;   // one thread per digit
+    int tile = 0, tile_end = 1;
+    uint32_t dnext = 0;  // RUNS: global start of the next tile's run of digit b
+    if (RUNS) {
+        tile = (int)(blockIdx.x * (run / RADIX_TILE));
+        tile_end = (int)min((int64_t)tile + run / RADIX_TILE, (n + RADIX_TILE - 1) / RADIX_TILE);
+        dnext = radix_block_scan(b < bins ? hist[b] : 0u, R.wsum);
+        if (b < bins) dnext += words[(int64_t)blockIdx.x * bins + b];
+        __syncthreads();
+    } else {
+        if (tid == 0) {
+            R.tile = (int)atomicAdd(tile_counter, 1u);
+            R.failed = 0;
         }
-        if (valid) {
-            int leader = __ffs(peers) - 1;
+        __syncthreads();
+        tile = R.tile;
+        tile_end = tile + 1;
+    }
+    for (; tile < tile_end; tile++) {
+        for (int i = tid; i < RADIX_WARPS * RADIX_MAX_BINS; i += RADIX_THREADS) (&R.wh[0][0])[i] = 0u;
+        __syncthreads();
+        const int64_t tbase = (int64_t)tile * RADIX_TILE;
+        const int64_t wbase = tbase + (int64_t)warp * (32 * RADIX_ITEMS);
+        const int tcount = (int)min((int64_t)RADIX_TILE, n - tbase);
+        uint32_t k[RADIX_ITEMS], v[RADIX_ITEMS], r[RADIX_ITEMS];
+#pragma unroll
+        for (int j = 0; j < RADIX_ITEMS; j++) {
+            int64_t gi = wbase + j * 32 + lane;
+            bool valid = gi < n;
+            unsigned vm = __ballot_sync(0xffffffffu, valid);
+            k[j] = valid ? keys_in[gi] : 0u;
+            v[j] = valid ? (vals_in ? vals_in[gi] : (uint32_t)gi) : 0u;
+            r[j] = 0u;
+            // lanes holding the same digit: one ballot per digit bit (independent
+            // instructions, where a match has one long latency)
+            const uint32_t d = (k[j] >> shift) & dm;
+            unsigned peers = vm;
+#pragma unroll
+            for (int b = 0; b < RADIX_MAX_BITS; b++) {
+                if (b < bits) {
+                    const unsigned on = __ballot_sync(0xffffffffu, (d >> b) & 1u);
+                    peers &= ((d >> b) & 1u) ? on : ~on;
+                }
+            }
+            const int leader = valid ? __ffs(peers) - 1 : lane;
             uint32_t old = 0u;
-            if (lane == leader) {
+            if (valid && lane == leader) {
                 old = R.wh[warp][d];
                 R.wh[warp][d] = old + (uint32_t)__popc(peers);
             }
-            old = __shfl_sync(peers, old, leader);
+            // (the whole warp: a shuffle per group of equal digits runs the groups one after another)
+            old = __shfl_sync(0xffffffffu, old, leader);
             r[j] = old + (uint32_t)__popc(peers & lanemask_lt());
         }
-        __syncwarp();
-    }
-    __syncthreads();
-    // per digit: exclusive prefix over warps; the tile's count of the digit
-    constexpr int BPT = RADIX_MAX_BINS / RADIX_THREADS;   // bins per thread
-    static_assert(BPT >= 1, "a thread owns at least one bin");
-    uint32_t tot[BPT], part = 0;
-#pragma unroll
-    for (int q = 0; q < BPT; q++) {
-        const int b = tid * BPT + q;
-        uint32_t run = 0;
+        __syncthreads();
+        // exclusive prefix of each digit over warps; the tile's count
+        uint32_t total = 0;
         if (b < bins) {
 #pragma unroll
             for (int w = 0; w < RADIX_WARPS; w++) {
-                uint32_t c = R.wh[w][b];
-                R.wh[w][b] = run;
-                run += c;
+                const uint32_t c = R.wh[w][b];
+                R.wh[w][b] = total;
+                total += c;
             }
         }
-        tot[q] = run;
-        part += run;
-    }
-    // block-wide exclusive scan of the per-thread digit totals -> lbase
-    uint32_t incl = part;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-    }
-    if (lane == 31) R.wsum[warp] = incl;
-    __syncthreads();
-    uint32_t off = incl - part;
-    for (int w = 0; w < warp; w++) off += R.wsum[w];
-#pragma unroll
-    for (int q = 0; q < BPT; q++) {
-        const int b = tid * BPT + q;
-        if (b < bins) R.lbase[b] = off;
-        off += tot[q];
-    }
-    __syncthreads();
-    // stage the tile in digit order
-#pragma unroll
-    for (int j = 0; j < RADIX_ITEMS; j++) {
-        int64_t gi = wbase + j * 32 + lane;
-        if (gi < n) {
-            const uint32_t d = (k[j] >> shift) & dm;
-            const uint32_t lp = R.lbase[d] + R.wh[warp][d] + r[j];
-            R.key[lp] = k[j];
-            R.val[lp] = v[j];
+        if (RUNS) {
+            if (b < bins) R.dbase[b] = dnext;
+            dnext += total;
+        } else if (tile == 0) {
+            const uint32_t base = radix_block_scan(b < bins ? hist[b] : 0u, R.wsum);
+            if (b < bins) {
+                ((volatile uint32_t*)words)[b] = whole << WORD_SHIFT | (base + total);
+                R.dbase[b] = base;
+            }
+            __syncthreads();
+        } else if (b < bins) {
+            ((volatile uint32_t*)words)[tile * bins + b] = part << WORD_SHIFT | total;
         }
-    }
-    __syncthreads();
-    // write out: slot i of the staged tile goes to dbase[d] + (i - lbase[d])
-    for (int i = tid; i < tcount; i += RADIX_THREADS) {
-        const uint32_t kk = R.key[i];
-        const uint32_t d = (kk >> shift) & dm;
-        const uint32_t p = R.dbase[d] + ((uint32_t)i - R.lbase[d]);
-        if (keys_out) keys_out[p] = kk;
-        vals_out[p] = R.val[i];
+        const uint32_t lb = radix_block_scan(total, R.wsum);
+        if (b < bins) R.lbase[b] = lb;
+        __syncthreads();
+        // stage the tile in digit order
+#pragma unroll
+        for (int j = 0; j < RADIX_ITEMS; j++) {
+            int64_t gi = wbase + j * 32 + lane;
+            if (gi < n) {
+                const uint32_t d = (k[j] >> shift) & dm;
+                const uint32_t lp = R.lbase[d] + R.wh[warp][d] + r[j];
+                R.key[lp] = k[j];
+                R.val[lp] = v[j];
+            }
+        }
+        if (!RUNS && tile != 0 && b < bins) {
+            uint32_t sum = 0;   // keys of lower digits, and of b in the tiles before
+            long long polls = 0;
+            bool found = false;
+            for (int t = tile - 1; !found;) {
+                uint32_t w[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) w[u] = t - u >= 0 ? ((volatile uint32_t*)words)[(t - u) * bins + b] : 0u;
+                int seen = 0;
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const unsigned st = w[u] >> WORD_SHIFT;
+                    if (found || seen != u || (st != part && st != whole)) continue;
+                    sum += w[u] & ((1u << WORD_SHIFT) - 1u);
+                    seen++;
+                    found = st == whole;
+                }
+                t -= seen;
+                if (seen == 0 && ++polls > SCAN_SPIN_LIMIT) {
+                    raise_status(status, ST_TIMEOUT);
+                    R.failed = 1;
+                    break;
+                }
+            }
+            ((volatile uint32_t*)words)[tile * bins + b] = whole << WORD_SHIFT | (sum + total);
+            R.dbase[b] = sum;
+        }
+        __syncthreads();
+        if (!RUNS && R.failed) return;
+        // write out: slot i of the staged tile goes to dbase[d] + (i - lbase[d])
+        for (int i = tid; i < tcount; i += RADIX_THREADS) {
+            const uint32_t kk = R.key[i];
+            const uint32_t d = (kk >> shift) & dm;
+            const uint32_t p = R.dbase[d] + ((uint32_t)i - R.lbase[d]);
+            if (keys_out) keys_out[p] = kk;
+            vals_out[p] = R.val[i];
+        }
+        __syncthreads();
     }
 }
 
@@ -420,9 +534,8 @@ void grid_dims(const float aabb[6], int64_t n, int desired, int dims[3], float* 
 }
 
 void grid_scratch_sizes(int64_t n, int64_t max_keys, size_t* hist_elems, size_t* scan_ws_bytes) {
-    int64_t tiles = std::max<int64_t>(1, (n + RADIX_TILE - 1) / RADIX_TILE);
-    *hist_elems = (size_t)RADIX_MAX_BINS * tiles;
-    *scan_ws_bytes = std::max(scan_workspace_bytes((int64_t)RADIX_MAX_BINS * tiles), scan_workspace_bytes(max_keys + 1));
+    *hist_elems = radix_hist_elems(n);
+    *scan_ws_bytes = scan_workspace_bytes(max_keys + 1);
 }
 
 int grid_auto_subdiv(uint32_t max_count, int k_hint) {
@@ -517,42 +630,64 @@ cudaError_t grid_sort(GridBuffers& B, const float aabb[6], GridPlan& plan, int S
     return e;
 }
 
+// per-pass digit totals, tile counters, and a word per (block, digit)
 size_t radix_hist_elems(int64_t n) {
-    return (size_t)RADIX_MAX_BINS * (size_t)std::max<int64_t>(1, (n + RADIX_TILE - 1) / RADIX_TILE);
+    const int64_t tiles = std::min<int64_t>(std::max<int64_t>(1, (n + RADIX_TILE - 1) / RADIX_TILE), RADIX_BLOCKS);
+    return RADIX_MAX_PASSES * RADIX_MAX_BINS + RADIX_MAX_PASSES + RADIX_MAX_BINS * (size_t)tiles;
 }
 
 // Stable LSD radix sort of n keys below 2^key_bits, digits of equal width <= 9 bits.
+// Up to RADIX_BLOCKS tiles (1.8M keys) a pass is one launch, its tiles looking
+// back over each other; beyond, three launches (counts, offsets, scatter): with
+// more tiles than resident blocks each wave of them starts together and most of
+// the look-back is waiting (10M keys: 0.23 ms a pass).
 cudaError_t radix_sort_u32(const RadixBuffers& B, const uint32_t* keys_in, const uint32_t* vals_in, int64_t n,
                            int key_bits, bool want_keys, const uint32_t** keys_sorted, const uint32_t** vals_sorted,
                            int* launches, cudaStream_t st) {
     cudaError_t e;
     const int bits = std::min(std::max(key_bits, 1), 32);
     const int passes = (bits + RADIX_MAX_BITS - 1) / RADIX_MAX_BITS;
-    const int width = (bits + passes - 1) / passes;
-    const int tiles = (int)((n + RADIX_TILE - 1) / RADIX_TILE);
-    const int64_t hist_n = ((int64_t)1 << width) * tiles;
+    const int width = (bits + passes - 1) / passes, bins = 1 << width;
+    const int64_t tiles = (n + RADIX_TILE - 1) / RADIX_TILE;
+    const bool runs = tiles > RADIX_BLOCKS;
+    const int64_t run = (runs ? (tiles + RADIX_BLOCKS - 1) / RADIX_BLOCKS : 1) * RADIX_TILE;
+    const int blocks = (int)((n + run - 1) / run);
+    uint32_t* hist = B.hist;
+    unsigned* counters = hist + RADIX_MAX_PASSES * RADIX_MAX_BINS;
+    uint32_t* words = counters + RADIX_MAX_PASSES;
+    auto kernel = runs ? k_radix_pass<true> : k_radix_pass<false>;
+    if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RadixSmem))) != cudaSuccess)
+        return e;
+    if (!runs) {
+        const size_t clear = RADIX_MAX_PASSES * RADIX_MAX_BINS + RADIX_MAX_PASSES + (size_t)blocks * bins;
+        if ((e = cudaMemsetAsync(hist, 0, clear * 4, st)) != cudaSuccess) return e;
+        k_radix_hist<<<blocks, RADIX_THREADS, 0, st>>>(keys_in, n, width, passes, hist);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        *launches += 1;
+    }
     const uint32_t* kin = keys_in;
     const uint32_t* vin = vals_in;
-    if ((e = cudaFuncSetAttribute(k_radix_downsweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(RadixSmem))) !=
-        cudaSuccess)
-        return e;
     for (int p = 0; p < passes; p++) {
-        const int shift = width * p;
         const bool last = p == passes - 1;
         uint32_t* kout = (last && !want_keys) ? nullptr : B.keys[p & 1];
         uint32_t* vout = B.vals[p & 1];
-        k_radix_upsweep<<<tiles, RADIX_THREADS, 0, st>>>(kin, n, shift, width, B.hist, tiles);
+        uint32_t* h = hist + p * RADIX_MAX_BINS;
+        if (runs) {
+            k_radix_count<<<blocks, RADIX_THREADS, 0, st>>>(kin, n, run, width * p, bins, words);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            k_radix_offsets<<<bins, RADIX_THREADS, 0, st>>>(words, blocks, bins, h);
+            if ((e = cudaGetLastError()) != cudaSuccess) return e;
+            *launches += 2;
+        }
+        kernel<<<blocks, RADIX_THREADS, sizeof(RadixSmem), st>>>(kin, vin, n, run, width, p, h, words, counters + p, kout, vout,
+                                                                 B.status);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        if ((e = scan_u32(B.hist, B.hist, hist_n, 0, nullptr, B.scan_ws, B.status, st)) != cudaSuccess) return e;
-        k_radix_downsweep<<<tiles, RADIX_THREADS, sizeof(RadixSmem), st>>>(kin, vin, n, shift, width, B.hist, tiles,
-                                                                           kout, vout);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        *launches += 1;
         kin = kout;
         vin = vout;
     }
     if (keys_sorted) *keys_sorted = kin;
     if (vals_sorted) *vals_sorted = vin;
-    *launches += 3 * passes;
     return cudaSuccess;
 }
 
@@ -561,7 +696,7 @@ cudaError_t radix_sort_u32(const RadixBuffers& B, const uint32_t* keys_in, const
 cudaError_t radix_and_gather(GridBuffers& B, int64_t n, int64_t key_space, int* launches, cudaStream_t st) {
     int bits = 1;
     while (bits < 32 && ((uint64_t)1 << bits) < (uint64_t)key_space) bits++;
-    RadixBuffers RB{{B.keys[0], B.keys[1]}, {B.vals[0], B.vals[1]}, B.hist, B.scan_ws, B.status};
+    RadixBuffers RB{{B.keys[0], B.keys[1]}, {B.vals[0], B.vals[1]}, B.hist, B.status};
     const uint32_t* order = nullptr;
     cudaError_t e = radix_sort_u32(RB, B.cid, nullptr, n, bits, false, nullptr, &order, launches, st);
     if (e != cudaSuccess) return e;

@@ -33,7 +33,7 @@ struct GridBuffers {
     uint32_t* keys[2];    // n each
     uint32_t* vals[2];    // n each
     uint32_t* counts2;    // cells of the re-grid resolution (count scratch)
-    uint32_t* hist;       // 512 * tiles
+    uint32_t* hist;       // radix_hist_elems(n)
     void* scan_ws;
     uint32_t* small;      // 16 u32 of device scratch (max count, totals)
     uint32_t* host_words = nullptr;   // 2 pinned host words the count maxima are read into (else the stack)
@@ -87,12 +87,11 @@ cudaError_t grid_multi(GridBuffers& B, const GridMulti& M, int* launches, cudaSt
 cudaError_t radix_and_gather(GridBuffers& B, int64_t n, int64_t key_space, int* launches, cudaStream_t st);
 
 // Scratch of a stand-alone radix sort: keys / vals ping-pong buffers (n each),
-// hist (radix_hist_elems(n)), scan workspace (scan_workspace_bytes(hist elems)).
+// hist (radix_hist_elems(n)).
 struct RadixBuffers {
     uint32_t* keys[2];
     uint32_t* vals[2];
     uint32_t* hist;
-    void* scan_ws;
     unsigned* status;
 };
 size_t radix_hist_elems(int64_t n);

@@ -242,7 +242,7 @@ inline unsigned blocks_of(int64_t n, int t) { return (unsigned)((n + t - 1) / t)
 
 // scratch carve-up (byte offsets, 256-aligned)
 struct Layout {
-    size_t cb, codes, keys0, keys1, vals0, vals1, hist, scan, child, range, pint, pleaf, arrived, ibox, lbox, cost,
+    size_t cb, codes, keys0, keys1, vals0, vals1, hist, child, range, pint, pleaf, arrived, ibox, lbox, cost,
         isleaf, total;
 };
 inline size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -259,7 +259,6 @@ Layout layout(int n) {
     L.vals0 = take(N * 4);
     L.vals1 = take(N * 4);
     L.hist = take(hist * 4);
-    L.scan = take(scan_workspace_bytes((int64_t)hist));
     L.child = take(2 * N * 4);
     L.range = take(2 * N * 4);
     L.pint = take(N * 4);
@@ -353,7 +352,7 @@ cudaError_t lbvh_build(const float* tri_pos, int ntri, float pad, float4* nodes,
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     RadixBuffers RB{{reinterpret_cast<uint32_t*>(base + L.keys0), reinterpret_cast<uint32_t*>(base + L.keys1)},
                     {reinterpret_cast<uint32_t*>(base + L.vals0), reinterpret_cast<uint32_t*>(base + L.vals1)},
-                    reinterpret_cast<uint32_t*>(base + L.hist), base + L.scan, status};
+                    reinterpret_cast<uint32_t*>(base + L.hist), status};
     const uint32_t* skeys = nullptr;
     const uint32_t* order = nullptr;
     if ((e = radix_sort_u32(RB, codes, nullptr, n, 30, true, &skeys, &order, launches, st)) != cudaSuccess) return e;
