@@ -73,7 +73,7 @@ std::vector<DevBuf*> all_buffers(pm_ctx* ctx) {
     for (auto& m : ctx->maps)
         for (DevBuf* b : {&m.pos, &m.dir, &m.pow, &m.starts, &m.sizes, &m.gpos, &m.gdir, &m.gpow, &m.cid, &m.keys0,
                           &m.keys1, &m.vals0, &m.vals1, &m.hist, &m.scan_ws, &m.small, &m.key_counts,
-                          &m.key_starts, &m.counts2, &m.rec})
+                          &m.key_starts, &m.counts2, &m.rank, &m.rec})
             v.push_back(b);
     return v;
 }
@@ -1019,7 +1019,7 @@ int grid_issue(pm_ctx* ctx, int map, const pm_grid_opts* o, const float* aabb, G
     B.cid = P<uint32_t>(m.cid);
     B.keys[0] = P<uint32_t>(m.keys0); B.keys[1] = P<uint32_t>(m.keys1);
     B.vals[0] = P<uint32_t>(m.vals0); B.vals[1] = P<uint32_t>(m.vals1);
-    B.host_words = ctx->hbuf + 4;
+    B.host_words = ctx->hbuf + 8;
     B.small = P<uint32_t>(m.small);
     B.counts2 = P<uint32_t>(m.counts2);
     B.status = P<unsigned>(ctx->status);
@@ -1033,11 +1033,13 @@ int grid_issue(pm_ctx* ctx, int map, const pm_grid_opts* o, const float* aabb, G
     grid_scratch_sizes(n, keys, &hist_elems, &scan_ws);
     ENSURE(m.hist, hist_elems * 4);
     ENSURE(m.scan_ws, scan_ws);
-    ENSURE(m.key_counts, (size_t)keys * 4);
+    ENSURE(m.key_counts, ((size_t)std::max<uint32_t>(plan.full_cells, 1) * S * S * S + 1) * 4);
+    ENSURE(m.rank, (size_t)plan.cells * 4);
     ENSURE(m.key_starts, (size_t)(keys + 1) * 4);
     B.hist = P<uint32_t>(m.hist);
     B.scan_ws = m.scan_ws.p;
     B.key_counts = P<uint32_t>(m.key_counts);
+    B.rank = P<uint32_t>(m.rank);
     B.key_starts = P<uint32_t>(m.key_starts);
     CK(grid_sort(B, box, plan, S, ctx->st));
     ctx->launches += plan.launches;

@@ -34,7 +34,7 @@ struct MapState {
     float aabb[6] = {0, 0, 0, 0, 0, 0};
     int S = 1;
     DevBuf starts, sizes, gpos, gdir, gpow, key_counts, key_starts;
-    DevBuf cid, keys0, keys1, vals0, vals1, hist, scan_ws, small, counts2;
+    DevBuf cid, keys0, keys1, vals0, vals1, hist, scan_ws, small, counts2, rank;
 };
 
 }  // namespace pm

@@ -26,17 +26,18 @@ struct GridBuffers {
     float4* gpos;         // sorted: xyz + source index bits in w
     float* gdir;          // sorted: 3 floats per photon
     float* gpow;          // sorted: 3 floats per photon
-    uint32_t* key_counts; // cells * S^3 (sub-cell counts)
+    uint32_t* key_counts; // scratch: cells with photons * S^3 + 1 (grid_multi: all keys)
     uint32_t* key_starts; // cells * S^3 + 1 (exclusive scan, total last)
     // scratch
     uint32_t* cid;        // n
     uint32_t* keys[2];    // n each
     uint32_t* vals[2];    // n each
     uint32_t* counts2;    // cells of the re-grid resolution (count scratch)
+    uint32_t* rank = nullptr;   // cells (grid_sort)
     uint32_t* hist;       // radix_hist_elems(n)
     void* scan_ws;
     uint32_t* small;      // 16 u32 of device scratch (max count, totals)
-    uint32_t* host_words = nullptr;   // 2 pinned host words the count maxima are read into (else the stack)
+    uint32_t* host_words = nullptr;   // 4 pinned host words the counts are read into (else the stack)
     unsigned* status;
 };
 
@@ -45,6 +46,8 @@ struct GridPlan {
     float cell;
     int64_t cells;
     uint32_t max_count;   // photons in the fullest cell of the chosen grid
+    uint32_t full_cells;  // its cells that hold photons
+    const uint32_t* counts;   // device: its photons per cell
     int launches;         // kernels launched by grid_count + grid_sort
 };
 
