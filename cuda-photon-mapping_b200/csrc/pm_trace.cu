@@ -52,18 +52,36 @@ constexpr int TRACE_REFILL = 8;          // default for KParams::refill (12 lane
 // lanes' hits back (10M photons: 3.85 -> 3.80 ms; 100M-photon stress scene
 // -4 %; 2, 4, 8 and 12 lanes measure the same or slower).
 constexpr int TRACE_CUT = 6;
+// Lanes whose rejection loop has to try again that are enough for another try at
+// once; fewer wait until the warp next leaves its traversal (8: the waiting
+// lanes thin the traversal, 3.45 ms per 10M photons instead of 3.18; 1: 3.22).
+// A launch of few paths ends with its longest one and tries at once (100K
+// photons: 0.18 ms, 0.20 with 3).
+constexpr int SAMPLE_AGAIN = 3;
+constexpr int64_t SAMPLE_AGAIN_PATHS = 4 * (int64_t)148 * TRACE_MIN_BLOCKS * TRACE_THREADS;
+inline int sample_again(int64_t npaths) { return npaths < SAMPLE_AGAIN_PATHS ? 1 : SAMPLE_AGAIN; }
 
 enum { DIF = 0, SPEC = 1, ABSORB = 2, REFR = 3, NONE = 4 };
 
-// The random stream of a photon path, two forms of the same Philox-4x32-10
-// stream (pm_device.cuh's Stream: draw i is word (i & 3) of Philox(counter =
-// (i >> 2, path_lo, path_hi, tag), key = seed)):
+// Lane states of k_trace.
+enum { L_IDLE = 0, L_RAY = 1, L_TRACE = 2, L_HIT = 3, L_DONE = 4, L_START = 5, L_BOUNCE = 6 };
+
+// The random stream of a photon path: draw i is word (i & 3) of
+// Philox-4x32-10(counter = (i >> 2, path_lo, path_hi, tag), key = seed)
+// (pm_device.cuh's Stream).  A lane keeps its draw counter and the block of
+// four words that its next draw lies in.  Draws are taken through a window
+// (open_window / close_window): all lanes that draw compute their next block
+// together, once per step, and read up to four words across the two.  Lanes stand at
+// different words of their blocks, so a block computed when a lane runs out
+// made nearly every draw of a warp compute one, a quarter of the lanes active.
+// With the rejection loops' tries of new paths and of bounces made together
+// (sample_try): 10M photons 3.27 -> 3.18 ms, 1M + 120K caustic ones 2.12 -> 2.01.
+// Two forms:
 //  * ParamStream (k_trace): the launch's tag and the seed's ten round keys
-//    (rk0 / rk1) are read from the kernel parameters, so a lane holds only
-//    its path index, draw counter and the current block of four words, and
-//    a Philox round takes no key additions (10M photons: 4.00 -> 3.85 ms);
+//    (rk0 / rk1) are read from the kernel parameters, so a Philox round takes
+//    no key additions and a lane no registers for the key;
 //  * RegStream (k_trace_multi, whose lanes trace different instances, each
-//    with its own seed): pm_device.cuh's Stream, keys in registers.
+//    with its own seed): keys in registers.
 struct KParams;
 struct ParamStream {
     uint32_t plo, phi, n;
@@ -71,19 +89,49 @@ struct ParamStream {
     __device__ __forceinline__ void init(const KParams&, uint64_t path) {
         plo = (uint32_t)path; phi = (uint32_t)(path >> 32); n = 0;
     }
-    __device__ __forceinline__ float next(const KParams& P);
+    __device__ __forceinline__ uint4 block(const KParams& P, uint32_t i) const;
 };
 struct RegStream {
-    Stream s;
+    uint32_t plo, phi, n;
+    uint4 buf;
+    uint32_t k0, k1, tag;
     __device__ __forceinline__ void init(const KParams& P, uint64_t path);
-    __device__ __forceinline__ float next(const KParams&) { return s.next(); }
+    __device__ __forceinline__ uint4 block(const KParams&, uint32_t i) const {
+        return philox10(make_uint4(i, plo, phi, tag), k0, k1);
+    }
 };
+
+// The next four words of a stream (at least as many as one step draws) and the
+// block that they may end in.
+struct Window {
+    uint4 nb;
+    uint32_t w0, w1, w2, w3;
+};
+template <class St>
+__device__ __forceinline__ Window open_window(const St& st, const KParams& P) {
+    Window W;
+    const uint32_t p = st.n & 3u;
+    W.nb = st.block(P, (st.n + 3u) >> 2);   // the block after buf (p != 0: buf holds words p .. 3 still)
+    W.w0 = p == 0u ? W.nb.x : p == 1u ? st.buf.y : p == 2u ? st.buf.z : st.buf.w;
+    W.w1 = p == 0u ? W.nb.y : p == 1u ? st.buf.z : p == 2u ? st.buf.w : W.nb.x;
+    W.w2 = p == 0u ? W.nb.z : p == 1u ? st.buf.w : p == 2u ? W.nb.x : W.nb.y;
+    W.w3 = p == 0u ? W.nb.w : p == 1u ? W.nb.x : p == 2u ? W.nb.y : W.nb.z;
+    return W;
+}
+// `used` (<= 4) of the window's words are drawn
+template <class St>
+__device__ __forceinline__ void close_window(St& st, const Window& W, uint32_t used) {
+    const uint32_t p = st.n & 3u;
+    if (p == 0u || p + used > 4u) st.buf = W.nb;
+    st.n += used;
+}
 
 template <class St>
 struct Lane {
     St st;
-    Ray ray;
-    int bounce;
+    Ray ray;                // L_START: o = the ray's origin, d = the light's normal;
+                            // L_BOUNCE: o = the hit point, d = its normal
+    int bounce;             // L_START: tries so far
     int ng, nc;             // photons stored so far (global / caustic)
     int diffuse_surfs;
     int last;
@@ -103,26 +151,25 @@ struct KParams {
     uint32_t* cnt_c;
     unsigned* status;
     int refill;             // lanes with a finished query that end a warp's traversal loop
+    int again;              // sample_again
     unsigned long long* work;   // work-counting launch: rays, BVH node visits, triangle tests (else null)
     uint32_t rk0[10], rk1[10];  // Philox round keys of seed: low / high word + round x (0x9E3779B9, 0xBB67AE85)
 };
 
-__device__ __forceinline__ float ParamStream::next(const KParams& P) {
-    if ((n & 3u) == 0u) {
-        uint4 c = make_uint4(n >> 2, plo, phi, P.tag);
+__device__ __forceinline__ uint4 ParamStream::block(const KParams& P, uint32_t i) const {
+    uint4 c = make_uint4(i, plo, phi, P.tag);
 #pragma unroll
-        for (int r = 0; r < 10; ++r) {   // philox10 of pm_device.cuh with the round keys precomputed
-            const uint32_t hi0 = __umulhi(0xD2511F53u, c.x), lo0 = 0xD2511F53u * c.x;
-            const uint32_t hi1 = __umulhi(0xCD9E8D57u, c.z), lo1 = 0xCD9E8D57u * c.z;
-            c = make_uint4(hi1 ^ c.y ^ P.rk0[r], lo1, hi0 ^ c.w ^ P.rk1[r], lo0);
-        }
-        buf = c;
+    for (int r = 0; r < 10; ++r) {   // philox10 of pm_device.cuh with the round keys precomputed
+        const uint32_t hi0 = __umulhi(0xD2511F53u, c.x), lo0 = 0xD2511F53u * c.x;
+        const uint32_t hi1 = __umulhi(0xCD9E8D57u, c.z), lo1 = 0xCD9E8D57u * c.z;
+        c = make_uint4(hi1 ^ c.y ^ P.rk0[r], lo1, hi0 ^ c.w ^ P.rk1[r], lo0);
     }
-    const uint32_t w = (n & 3u) == 0u ? buf.x : (n & 3u) == 1u ? buf.y : (n & 3u) == 2u ? buf.z : buf.w;
-    ++n;
-    return unit_from_u32(w);
+    return c;
 }
-__device__ __forceinline__ void RegStream::init(const KParams& P, uint64_t path) { s.init(P.seed, path, P.tag); }
+__device__ __forceinline__ void RegStream::init(const KParams& P, uint64_t path) {
+    plo = (uint32_t)path; phi = (uint32_t)(path >> 32); n = 0;
+    k0 = (uint32_t)P.seed; k1 = (uint32_t)(P.seed >> 32); tag = P.tag;
+}
 
 // the round keys of KParams::seed (philox10's key schedule)
 static void round_keys(KParams& P) {
@@ -135,39 +182,25 @@ static void round_keys(KParams& P) {
     }
 }
 
-// light point + cosine-weighted direction by rejection (PhotonTracing.cu:345-369)
+// light point of a new path (PhotonTracing.cu:345-369); its direction is found
+// by start_try
 template <class LaneT>
-__device__ __forceinline__ void start_path(const KParams& P, LaneT& L, int64_t path) {
+__device__ __forceinline__ void begin_path(const KParams& P, LaneT& L, int64_t path) {
     const DevScene& S = P.S;
     L.st.init(P, (uint64_t)path);
-    int k = (int)roundf(0 + L.st.next(P) * (float)(S.light_count - 1));
+    L.st.buf = L.st.block(P, 0u);
+    int k = (int)roundf(0 + unit_from_u32(L.st.buf.x) * (float)(S.light_count - 1));
     int tri = S.light_first + k;
-    float bx = L.st.next(P);
-    float by = 0.f + L.st.next(P) * ((1.f - bx) - 0.f);
+    float bx = unit_from_u32(L.st.buf.y);
+    float by = 0.f + unit_from_u32(L.st.buf.z) * ((1.f - bx) - 0.f);
+    L.st.n = 3u;
     float bz = 1.f - bx - by;
     const float* tp = S.tri_pos + 9 * (size_t)tri;
     const float* tn = S.tri_nrm + 9 * (size_t)tri;
     V3 point = vadd(vadd(vscale(ld3(tp), bx), vscale(ld3(tp + 3), by)), vscale(ld3(tp + 6), bz));
     V3 lnorm = vadd(vadd(vscale(ld3(tn), bx), vscale(ld3(tn + 3), by)), vscale(ld3(tn + 6), bz));
     L.ray.o = vadd(point, vscale(lnorm, 0.0001f));
-    float prob, dt;
-    V3 d;
-    int tries = 0;
-    do {
-        if (++tries > REJECT_LIMIT) {   // a light without a usable normal: end the path
-            raise_status(P.status, ST_BAD_INPUT);
-            L.ray.d = v3(0.f, 0.f, 0.f);
-            break;
-        }
-        d.x = -1.f + L.st.next(P) * 2.f;
-        d.y = -1.f + L.st.next(P) * 2.f;
-        d.z = -1.f + L.st.next(P) * 2.f;
-        d = vnorm_recip(d);
-        prob = L.st.next(P);
-        dt = vdot(d, lnorm);
-        if (dt < 0) { dt = -dt; d = vscale(d, -1.f); }
-    } while (prob > dt);
-    if (tries <= REJECT_LIMIT) L.ray.d = d;
+    L.ray.d = lnorm;
     L.bounce = 0;
     L.ng = L.nc = 0;
     L.diffuse_surfs = 0;
@@ -175,25 +208,40 @@ __device__ __forceinline__ void start_path(const KParams& P, LaneT& L, int64_t p
     L.sn = 0;
 }
 
-// Marsaglia disc, rejected into the hemisphere of n (Ray.cuh:16-56)
-template <class St>
-__device__ __forceinline__ Ray diffuse_bounce(V3 from, V3 n, St& st, const KParams& P) {
-    V3 d;
-    do {
-        float x1, x2, s1, s2;
-        do {
-            x1 = -1.f + st.next(P) * 2.f;
-            x2 = -1.f + st.next(P) * 2.f;
-            s1 = x1 * x1;
-            s2 = x2 * x2;
-        } while (s1 + s2 >= 1);
-        float f = sqrtf(1.f - s1 - s2);
-        d = v3(2.f * x1 * f, 2.f * x2 * f, 1.f - 2.f * (s1 + s2));
-    } while (vdot(d, n) < 0);
-    Ray r;
-    r.d = vnorm_div(d);
-    r.o = vadd(from, vscale(r.d, 0.0001f));
-    return r;
+// One try of a rejection loop, for the lanes of a warp that sample; true: the
+// ray is set.  Light direction (start): cosine-weighted by rejection
+// (PhotonTracing.cu:345-369).  Diffuse bounce: Marsaglia disc, rejected into the
+// hemisphere of the normal (Ray.cuh:16-56).
+template <class LaneT>
+__device__ __forceinline__ bool sample_try(const KParams& P, LaneT& L, bool start) {
+    const Window W = open_window(L.st, P);
+    const float a = -1.f + unit_from_u32(W.w0) * 2.f, b = -1.f + unit_from_u32(W.w1) * 2.f;
+    if (start) {
+        if (++L.bounce > REJECT_LIMIT) {   // a light without a usable normal: end the path
+            raise_status(P.status, ST_BAD_INPUT);
+            L.ray.d = v3(0.f, 0.f, 0.f);
+            L.bounce = 0;
+            return true;
+        }
+        V3 d = vnorm_recip(v3(a, b, -1.f + unit_from_u32(W.w2) * 2.f));
+        const float prob = unit_from_u32(W.w3);
+        float dt = vdot(d, L.ray.d);
+        if (dt < 0) { dt = -dt; d = vscale(d, -1.f); }
+        close_window(L.st, W, 4u);
+        if (prob > dt) return false;
+        L.ray.d = d;
+        L.bounce = 0;
+        return true;
+    }
+    close_window(L.st, W, 2u);
+    const float s1 = a * a, s2 = b * b;
+    if (s1 + s2 >= 1) return false;
+    const float f = sqrtf(1.f - s1 - s2);
+    const V3 d = v3(2.f * a * f, 2.f * b * f, 1.f - 2.f * (s1 + s2));
+    if (vdot(d, L.ray.d) < 0) return false;
+    L.ray.d = vnorm_div(d);
+    L.ray.o = vadd(L.ray.o, vscale(L.ray.d, 0.0001f));
+    return true;
 }
 
 // Fresnel-Schlick with the integer powers written as products (PhotonTracing.cu:215-218)
@@ -206,10 +254,11 @@ __device__ __forceinline__ float schlick(float cosNL, float n1, float n2) {
     return f0 + (1.f - f0) * c5;
 }
 
-// the surface interaction of one bounce of lane L at hit h (PhotonTracing.cu:278-326);
-// returns false when the path ends
+// the surface interaction of one bounce of lane L at hit h (PhotonTracing.cu:278-326):
+// L_RAY (its next ray is set), L_BOUNCE (a diffuse bounce, its direction still to
+// be sampled) or L_IDLE (the path ends)
 template <class LaneT>
-__device__ __forceinline__ bool shade(const KParams& P, LaneT& L, const Hit& h, float* sior, int* sid, int64_t j) {
+__device__ __forceinline__ int shade(const KParams& P, LaneT& L, const Hit& h, float* sior, int* sid, int64_t j) {
     const DevScene& S = P.S;
     const int model = hit_model(S, h.tri);
     const Material m = load_mat(S, model);
@@ -219,6 +268,8 @@ __device__ __forceinline__ bool shade(const KParams& P, LaneT& L, const Hit& h, 
     float cosNL = vdot(vneg(L.ray.d), n);
     V3 mdiff = tri_albedo(S, h.tri, m);
 
+    const Window W = open_window(L.st, P);
+    uint32_t used = 0u;
     int dest;
     bool refr = false;
     if (m.opaque != 1.f) {
@@ -230,7 +281,8 @@ __device__ __forceinline__ bool shade(const KParams& P, LaneT& L, const Hit& h, 
         bool tir = critical_angle(S, n1, n2, cang) && cosNL <= cang;
         if (!tir) {
             float pr = 1.f - schlick(cosNL, n1, n2);
-            float e = L.st.next(P);
+            float e = unit_from_u32(W.w0);
+            used = 1u;
             refr = !(e > pr);
         }
     }
@@ -238,7 +290,8 @@ __device__ __forceinline__ bool shade(const KParams& P, LaneT& L, const Hit& h, 
         dest = REFR;
     } else {
         float max_lp = vmax3(P.power);
-        float e = 0.f + L.st.next(P) * (2.f - 0.f);
+        float e = 0.f + unit_from_u32(used ? W.w1 : W.w0) * (2.f - 0.f);
+        used++;
         float pd = vmax3(vmul(mdiff, P.power)) / max_lp;
         if (e <= pd) dest = DIF;
         else {
@@ -246,6 +299,8 @@ __device__ __forceinline__ bool shade(const KParams& P, LaneT& L, const Hit& h, 
             dest = (e <= pd + ps) ? SPEC : ABSORB;
         }
     }
+
+    close_window(L.st, W, used);
 
     Ray nr;
     nr.o = v3(0.f, 0.f, 0.f); nr.d = v3(0.f, 0.f, 0.f);
@@ -276,17 +331,15 @@ __device__ __forceinline__ bool shade(const KParams& P, LaneT& L, const Hit& h, 
         nr = ray_reflect(L.ray, ip, n);
     }
     if (dest == DIF) {
-        nr = diffuse_bounce(ip, n, L.st, P);
+        nr.o = ip;
+        nr.d = n;
         L.diffuse_surfs++;
     }
     L.last = dest;
-    if (dest == ABSORB || !alive) return false;
+    if (dest == ABSORB || !alive) return L_IDLE;
     L.ray = nr;
-    return true;
+    return dest == DIF ? L_BOUNCE : L_RAY;
 }
-
-// Lane states of k_trace.
-enum { L_IDLE = 0, L_RAY = 1, L_TRACE = 2, L_HIT = 3, L_DONE = 4 };
 
 // Persistent photon tracer.  Each lane runs a small state machine:
 //   IDLE  -> takes the next path of the batch (RAY) or finds none (DONE);
@@ -328,14 +381,18 @@ k_trace(KParams P) {
                 const unsigned long long mine = base + (unsigned long long)__popc(m & lanemask_lt());
                 if ((int64_t)mine < P.npaths) {
                     j = (int64_t)mine;
-                    start_path(P, L, P.p0 + j);
-                    state = L_RAY;
+                    begin_path(P, L, P.p0 + j);
+                    state = L_START;
                 } else {
                     state = L_DONE;
                 }
             }
         }
         if (__all_sync(0xffffffffu, state == L_DONE)) break;
+        while (true) {
+            if (state >= L_START && sample_try(P, L, state == L_START)) state = L_RAY;
+            if (__popc(__ballot_sync(0xffffffffu, state >= L_START)) < P.again) break;
+        }
         if (state == L_RAY) {
             trav_init(T, L.ray.o, L.ray.d, stack);
             if (COUNT) rays++;
@@ -344,7 +401,7 @@ k_trace(KParams P) {
         while (true) {
             const bool tr = state == L_TRACE;
             if (!__any_sync(0xffffffffu, tr)) break;
-            if (__popc(__ballot_sync(0xffffffffu, state == L_HIT)) >= P.refill) break;
+            if (__popc(__ballot_sync(0xffffffffu, state == L_HIT || state >= L_START)) >= P.refill) break;
             if (tr && trav_step<TRACE_CUT>(P.S, T, L.ray.o, L.ray.d, stack, work)) state = L_HIT;
         }
         if (state == L_HIT) {
@@ -353,15 +410,15 @@ k_trace(KParams P) {
             if (r == TRAV_AGAIN) {
                 state = L_TRACE;
             } else {
-                const bool alive = r == TRAV_HIT && shade(P, L, h, sior, sid, j);
+                const int next = r == TRAV_HIT ? shade(P, L, h, sior, sid, j) : L_IDLE;
                 L.bounce++;
-                if (!alive || L.bounce > P.max_bounces - 1) {
+                if (next == L_IDLE || L.bounce > P.max_bounces - 1) {
                     P.cnt_g[j] = (uint32_t)L.ng;
                     P.cnt_c[j] = (uint32_t)L.nc;
                     j = -1;
                     state = L_IDLE;
                 } else {
-                    state = L_RAY;
+                    state = next;
                 }
             }
         }
@@ -395,7 +452,7 @@ __device__ __forceinline__ int find_instance(const int64_t* __restrict__ off, in
 
 __global__ void __launch_bounds__(TRACE_THREADS, TRACE_MIN_BLOCKS)
 k_trace_multi(const KParams* __restrict__ tab, const int64_t* __restrict__ off, int ninst, int64_t total,
-              unsigned long long* counter, int refill) {
+              unsigned long long* counter, int refill, int again) {
     const int lane = threadIdx.x & 31;
     Lane<RegStream> L;
     Trav T;
@@ -421,8 +478,8 @@ k_trace_multi(const KParams* __restrict__ tab, const int64_t* __restrict__ off, 
                     j = (int64_t)mine;
                     inst = find_instance(off, ninst, j);
                     const KParams& P = tab[inst];
-                    start_path(P, L, P.p0 + (j - __ldg(off + inst)));
-                    state = L_RAY;
+                    begin_path(P, L, P.p0 + (j - __ldg(off + inst)));
+                    state = L_START;
                 } else {
                     state = L_DONE;
                 }
@@ -430,6 +487,10 @@ k_trace_multi(const KParams* __restrict__ tab, const int64_t* __restrict__ off, 
         }
         if (__all_sync(0xffffffffu, state == L_DONE)) break;
         const KParams& P = tab[inst];
+        while (true) {
+            if (state >= L_START && sample_try(P, L, state == L_START)) state = L_RAY;
+            if (__popc(__ballot_sync(0xffffffffu, state >= L_START)) < again) break;
+        }
         if (state == L_RAY) {
             trav_init(T, L.ray.o, L.ray.d, stack);
             state = L_TRACE;
@@ -437,7 +498,7 @@ k_trace_multi(const KParams* __restrict__ tab, const int64_t* __restrict__ off, 
         while (true) {
             const bool tr = state == L_TRACE;
             if (!__any_sync(0xffffffffu, tr)) break;
-            if (__popc(__ballot_sync(0xffffffffu, state == L_HIT)) >= refill) break;
+            if (__popc(__ballot_sync(0xffffffffu, state == L_HIT || state >= L_START)) >= refill) break;
             if (tr && trav_step<TRACE_CUT>(P.S, T, L.ray.o, L.ray.d, stack)) state = L_HIT;
         }
         if (state == L_HIT) {
@@ -446,15 +507,15 @@ k_trace_multi(const KParams* __restrict__ tab, const int64_t* __restrict__ off, 
             if (r == TRAV_AGAIN) {
                 state = L_TRACE;
             } else {
-                const bool alive = r == TRAV_HIT && shade(P, L, h, sior, sid, j);
+                const int next = r == TRAV_HIT ? shade(P, L, h, sior, sid, j) : L_IDLE;
                 L.bounce++;
-                if (!alive || L.bounce > P.max_bounces - 1) {
+                if (next == L_IDLE || L.bounce > P.max_bounces - 1) {
                     P.cnt_g[j] = (uint32_t)L.ng;
                     P.cnt_c[j] = (uint32_t)L.nc;
                     j = -1;
                     state = L_IDLE;
                 } else {
-                    state = L_RAY;
+                    state = next;
                 }
             }
         }
@@ -563,6 +624,7 @@ cudaError_t trace_multi_tables(const TraceMulti& M, const TraceInst* insts, cuda
         P.cnt_g = M.cnt_g; P.cnt_c = M.cnt_c;
         P.status = M.status;
         P.refill = M.refill > 0 ? std::min(M.refill, 32) : TRACE_REFILL;
+        P.again = 0;   // (a launch parameter)
         P.work = nullptr;
         round_keys(P);
     }
@@ -582,7 +644,7 @@ cudaError_t trace_multi(const TraceMulti& M, cudaStream_t st) {
     const int64_t grid = std::min<int64_t>(want, (int64_t)std::max(per_sm, 1) * M.sm_count);
     const int refill = M.refill > 0 ? std::min(M.refill, 32) : TRACE_REFILL;
     k_trace_multi<<<(unsigned)grid, TRACE_THREADS, 0, st>>>((const KParams*)M.table, M.path_off, M.ninst, M.total,
-                                                            M.path_counter, refill);
+                                                            M.path_counter, refill, sample_again(M.total));
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if ((e = scan_u32(M.cnt_g, M.scan_g, M.total, 0, M.totals, M.scan_ws, M.status, st)) != cudaSuccess) return e;
     const int64_t n = std::max<int64_t>(M.total, M.ninst);
@@ -605,6 +667,7 @@ cudaError_t trace_batch(TraceBatch& B, PhotonList& G, PhotonList& C, cudaStream_
     P.cnt_g = B.cnt_g; P.cnt_c = B.cnt_c;
     P.status = B.status;
     P.refill = B.refill > 0 ? std::min(B.refill, 32) : TRACE_REFILL;
+    P.again = sample_again(B.npaths);
     P.work = B.work;
     round_keys(P);
     int per_sm = 0;
