@@ -202,6 +202,22 @@ int render_checks(pm_ctx* ctx, const pm_camera* cam, const pm_render_opts* o) {
     return PM_OK;
 }
 
+namespace {
+// the columns [c0, c1] and rows [r0, r1] that cover the pixels [i0, i1) of eye_pixel's order
+void eye_block_rect(int64_t i0, int64_t i1, int W, int H, int& c0, int& c1, int& r0, int& r1) {
+    const int64_t band = 4 * (int64_t)W;
+    r0 = (int)(i0 / band) * 4;
+    r1 = std::min((int)((i1 - 1) / band) * 4 + 3, H - 1);
+    c0 = 0;
+    c1 = W - 1;
+    const int64_t a = i0 % band, z = a + (i1 - i0);   // one band's whole tiles: their columns
+    if (r0 + 3 == r1 && z <= 4 * (int64_t)(W & ~31)) {
+        c0 = (int)(a >> 7) * 32;
+        c1 = (int)((z - 1) >> 7) * 32 + 31;
+    }
+}
+}  // namespace
+
 int64_t eye_block_order(const pm_ctx* ctx, const pm_camera* cam, std::vector<int>& order) {
     const int W = cam->width, H = cam->height;
     const int64_t npx = (int64_t)W * H, nb = eye_blocks(npx), T = eye_threads();
@@ -258,15 +274,11 @@ int64_t eye_block_order(const pm_ctx* ctx, const pm_camera* cam, std::vector<int
     std::vector<int> rest;
     rest.reserve((size_t)nb);
     for (int64_t b = 0; b < nb; b++) {
-        const int64_t p0 = b * T, p1 = std::min(p0 + T - 1, npx - 1);
-        const int r0 = (int)(p0 / W), r1 = (int)(p1 / W);
+        int c0, c1, r0, r1;
+        eye_block_rect(b * T, std::min(b * T + T, npx), W, H, c0, c1, r0, r1);
         bool hot = false;
-        for (const Rect& r : rects) {
-            if (r1 < r.y0 || r0 > r.y1) continue;
-            if (r0 != r1) { hot = true; break; }
-            const int c0 = (int)(p0 % W), c1 = (int)(p1 % W);
-            if (c1 >= r.x0 && c0 <= r.x1) { hot = true; break; }
-        }
+        for (const Rect& r : rects)
+            if (r1 >= r.y0 && r0 <= r.y1 && c1 >= r.x0 && c0 <= r.x1) { hot = true; break; }
         (hot ? order : rest).push_back((int)b);
     }
     const int64_t first = (int64_t)order.size();
@@ -1290,10 +1302,13 @@ int render_eye_launch(pm_ctx* ctx, const pm_camera* cam, const pm_render_opts* o
     int64_t nblocks = -1;
     if (y0 < y1) {
         // the band's blocks, in the full order's (slow blocks first)
-        const int64_t T = eye_threads(), lo = (int64_t)y0 * cam->width, hi = (int64_t)y1 * cam->width;
+        const int64_t T = eye_threads();
         std::vector<int> band;
-        for (int b : ctx->h_eye_order)
-            if ((int64_t)b * T < hi && ((int64_t)b + 1) * T > lo) band.push_back(b);
+        for (int b : ctx->h_eye_order) {
+            int c0, c1, r0, r1;
+            eye_block_rect(b * T, std::min(b * T + T, F.npx), cam->width, cam->height, c0, c1, r0, r1);
+            if (r0 < y1 && r1 >= y0) band.push_back(b);
+        }
         ENSURE(ctx->eye_band, std::max<size_t>(band.size(), 1) * 4);
         if (!band.empty())
             CK(cudaMemcpyAsync(ctx->eye_band.p, band.data(), band.size() * 4, cudaMemcpyHostToDevice, st));
@@ -1302,7 +1317,8 @@ int render_eye_launch(pm_ctx* ctx, const pm_camera* cam, const pm_render_opts* o
         nblocks = (int64_t)band.size();
     }
     CK(cudaEventRecord(ctx->ev[4], st));
-    CK(eye_pass(F.S, F.cd, o->max_depth, R, P<unsigned>(ctx->status), st, order, nblocks));
+    CK(eye_pass(F.S, F.cd, o->max_depth, R, P<unsigned>(ctx->status), st, order, nblocks, y0 < y1 ? y0 : 0,
+                y0 < y1 ? y1 : cam->height));
     CK(cudaEventRecord(ctx->ev[5], st));
     ctx->launches += 1;
     return PM_OK;

@@ -346,8 +346,10 @@ __device__ __forceinline__ int trav_resolve(const DevScene& S, Trav& T, Hit& h, 
     return TRAV_HIT;
 }
 
-// Closest hit of one ray, both passes run to completion.
-static __device__ __noinline__ bool intersect(const DevScene& S, V3 o, V3 d, Hit& h) {
+// Closest hit of one ray, both passes run to completion.  Inlined: as a call it
+// reads the scene and writes the hit through local memory (eye pass at 1080p
+// 0.42 ms against 0.355, at 4K 1.46 against 1.27).
+__device__ __forceinline__ bool intersect(const DevScene& S, V3 o, V3 d, Hit& h) {
     LocalStack stack;
     Trav T;
     trav_init(T, o, d, stack);

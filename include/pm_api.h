@@ -225,11 +225,10 @@ int pm_camera_setup(const float position[3], const float direction[3], const flo
 int pm_render(pm_ctx* ctx, const pm_camera* cam, const pm_render_opts* opts, uint8_t* out_rgb8, float* out_radiance);
 
 /* The rows [y0, y1) of pm_render's frame (a pixel-row band; no counterpart in
- * the reference, whose frame is one launch): the eye pass runs only the pixel
- * blocks that meet those rows, so the band costs about its share of the
- * frame.  Pixels of the band are pm_render's bit for bit; every other pixel
- * of out_rgb8 / out_radiance holds 0 or, in the pixel blocks that straddle
- * the band's edges, pm_render's value.  For frames split over GPUs. */
+ * the reference, whose frame is one launch): the eye pass runs only the pixels
+ * of those rows, so the band costs about its share of the frame.  Pixels of
+ * the band are pm_render's bit for bit; every other pixel of out_rgb8 /
+ * out_radiance holds 0.  For frames split over GPUs. */
 int pm_render_rows(pm_ctx* ctx, const pm_camera* cam, const pm_render_opts* opts, int32_t y0, int32_t y1,
                    uint8_t* out_rgb8, float* out_radiance);
 
