@@ -65,7 +65,7 @@ std::vector<DevBuf*> all_buffers(pm_ctx* ctx) {
                               &ctx->scratch_pow, &ctx->req_a, &ctx->req_b, &ctx->req_c, &ctx->req_counter,
                               &ctx->px_base, &ctx->px_count, &ctx->est_g, &ctx->est_c, &ctx->status, &ctx->gws,
                               &ctx->cache_w32, &ctx->cache_w16, &ctx->cache_m, &ctx->cache_v, &ctx->cache_grad,
-                              &ctx->cache_loss, &ctx->est_mlp, &ctx->est_fb, &ctx->probe_pos, &ctx->probe_nrm,
+                              &ctx->est_mlp, &ctx->est_fb, &ctx->probe_pos, &ctx->probe_nrm,
                               &ctx->probe_req, &ctx->probe_est, &ctx->tile_flag, &ctx->learned_counts,
                               &ctx->fallback_list, &ctx->bvh_scratch, &ctx->tri_leaf, &ctx->eye_order, &ctx->rq_keys,
                               &ctx->rq_k0, &ctx->rq_k1, &ctx->rq_v0, &ctx->rq_v1, &ctx->rq_hist,
@@ -336,6 +336,7 @@ void pm_destroy(pm_ctx* ctx) {
     }
     if (ctx->frame_fork) cudaEventDestroy(ctx->frame_fork);
     if (ctx->hbuf) cudaFreeHost(ctx->hbuf);
+    if (ctx->hgrad) cudaFreeHost(ctx->hgrad);
     if (ctx->frame_done) cudaEventDestroy(ctx->frame_done);
     if (ctx->train_fork) cudaEventDestroy(ctx->train_fork);
     if (ctx->train_done) cudaEventDestroy(ctx->train_done);
@@ -378,22 +379,26 @@ MlpInputs cache_inputs(const float* pos, const float* nrm, int64_t n) {
     return in;
 }
 
-// loss and gradient of n samples into ctx->cache_grad (zeroed first); loss_out: mean squared error
+// Gradient and squared-error sum of n samples into ctx->cache_grad (zeroed
+// first; the sum behind the gradient).  read_loss: the sum is queued for
+// cache_loss_of, to be read once the stream has been waited for.
 int cache_backprop(pm_ctx* ctx, const float* pos, const float* nrm, const float* target, const float* weight,
-                   int64_t n, float* loss_out, cudaStream_t st) {
-    CK(cudaMemsetAsync(ctx->cache_grad.p, 0, (size_t)PM_CACHE_PARAMS * 4, st));
-    CK(cudaMemsetAsync(ctx->cache_loss.p, 0, 4, st));
+                   int64_t n, bool read_loss, cudaStream_t st) {
+    float* loss = P<float>(ctx->cache_grad) + PM_CACHE_PARAMS;
+    CK(cudaMemsetAsync(ctx->cache_grad.p, 0, (size_t)(PM_CACHE_PARAMS + 1) * 4, st));
     const float grad_scale = 2.f / (3.f * (float)n);
     CK(mlp_train(cache_net(ctx), cache_inputs(pos, nrm, n), target, weight, grad_scale, P<float>(ctx->cache_grad),
-                 P<float>(ctx->cache_loss), P<unsigned>(ctx->status), ctx->sm_count, st));
+                 loss, P<unsigned>(ctx->status), ctx->sm_count, st));
     ctx->launches += 1;
-    if (loss_out) {
-        float l = 0.f;
-        CK(cudaMemcpyAsync(&l, ctx->cache_loss.p, 4, cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
-        *loss_out = l / (3.f * (float)n);
-    }
+    if (read_loss) CK(cudaMemcpyAsync(ctx->hbuf + 4, loss, 4, cudaMemcpyDeviceToHost, st));
     return PM_OK;
+}
+
+// mean squared error of the last cache_backprop(read_loss) over n samples
+float cache_loss_of(const pm_ctx* ctx, int64_t n) {
+    float l;
+    std::memcpy(&l, ctx->hbuf + 4, 4);
+    return l / (3.f * (float)n);
 }
 
 uint64_t splitmix64(uint64_t& x) {
@@ -429,8 +434,7 @@ int pm_cache_init(pm_ctx* ctx, const pm_cache_opts* o) {
     ENSURE(ctx->cache_w16, (size_t)PM_CACHE_PARAMS * 2);
     ENSURE(ctx->cache_m, (size_t)PM_CACHE_PARAMS * 4);
     ENSURE(ctx->cache_v, (size_t)PM_CACHE_PARAMS * 4);
-    ENSURE(ctx->cache_grad, (size_t)PM_CACHE_PARAMS * 4);
-    ENSURE(ctx->cache_loss, 16);
+    ENSURE(ctx->cache_grad, (size_t)(PM_CACHE_PARAMS + 1) * 4);
     // He-uniform weights for the ReLU layers, a small output layer; padding zero
     std::vector<float> w(PM_CACHE_PARAMS, 0.f);
     uint64_t state = o->seed;
@@ -464,13 +468,15 @@ int pm_cache_train_step(pm_ctx* ctx, const float* pos, const float* nrm, const f
     if (n <= 0 || !pos || !nrm || !target) return fail(ctx, PM_ERR_INVALID, "cache train: n > 0 and sample arrays required");
     CK(cudaSetDevice(ctx->device));
     if (int rc = cache_fence(ctx)) return rc;
-    if (int rc = cache_backprop(ctx, pos, nrm, target, weight, n, out_loss, ctx->st)) return rc;
+    if (int rc = cache_backprop(ctx, pos, nrm, target, weight, n, out_loss != nullptr, ctx->st)) return rc;
     ctx->cache_step++;
     const pm_cache_opts& o = ctx->cache_opts;
     CK(mlp_adam(P<float>(ctx->cache_w32), P<__nv_bfloat16>(ctx->cache_w16), P<float>(ctx->cache_grad),
                 P<float>(ctx->cache_m), P<float>(ctx->cache_v), ctx->cache_step, o.lr, o.beta1, o.beta2, o.eps, ctx->st));
     ctx->launches += 1;
-    return check_status(ctx, "cache train");
+    const int rc = check_status(ctx, "cache train");
+    if (out_loss) *out_loss = cache_loss_of(ctx, n);
+    return rc;
 }
 
 int pm_cache_train_steps(pm_ctx* ctx, const float* pos, const float* nrm, const float* target, const float* weight,
@@ -503,7 +509,7 @@ int pm_cache_train_steps(pm_ctx* ctx, const float* pos, const float* nrm, const 
     for (int s = 0; s < steps; ++s) {
         if (off + b > n) off = 0;
         if (int rc = cache_backprop(ctx, pos + off * 3, nrm + off * 3, target + off * 3, weight ? weight + off : nullptr,
-                                    b, s + 1 == steps ? out_loss : nullptr, st))
+                                    b, out_loss && s + 1 == steps, st))
             return rc;
         ctx->cache_step++;
         CK(mlp_adam(P<float>(ctx->cache_w32), P<__nv_bfloat16>(ctx->cache_w16), P<float>(ctx->cache_grad),
@@ -519,7 +525,10 @@ int pm_cache_train_steps(pm_ctx* ctx, const float* pos, const float* nrm, const 
         // the steps' device status is reported by the next call that synchronises
         return PM_OK;
     }
-    return out_loss ? check_status(ctx, "cache train steps") : PM_OK;
+    if (!out_loss) return PM_OK;
+    const int rc = check_status(ctx, "cache train steps");
+    if (steps > 0) *out_loss = cache_loss_of(ctx, b);
+    return rc;
 }
 
 int pm_cache_gradient(pm_ctx* ctx, const float* pos, const float* nrm, const float* target, const float* weight,
@@ -529,11 +538,23 @@ int pm_cache_gradient(pm_ctx* ctx, const float* pos, const float* nrm, const flo
     if (n <= 0 || !pos || !nrm || !target) return fail(ctx, PM_ERR_INVALID, "cache gradient: n > 0 and sample arrays required");
     CK(cudaSetDevice(ctx->device));
     if (int rc = cache_fence(ctx)) return rc;
-    if (int rc = cache_backprop(ctx, pos, nrm, target, weight, n, out_loss, ctx->st)) return rc;
-    CK(cudaMemcpyAsync(out_grad_host, ctx->cache_grad.p, (size_t)PM_CACHE_PARAMS * 4, cudaMemcpyDeviceToHost, ctx->st));
+    // Gradient and loss come back as one copy into page-locked memory behind the
+    // kernel and are waited for together with the status (262144 samples: 131
+    // us a call, of which the kernel is 87; 160 with a wait for the loss, a copy into
+    // pageable memory and a wait for the status).  Without page-locked memory the
+    // gradient is copied straight to the caller's.
+    if (!ctx->hgrad && cudaHostAlloc((void**)&ctx->hgrad, (PM_CACHE_PARAMS + 1) * 4, cudaHostAllocDefault) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->hgrad = nullptr;
+    }
+    if (int rc = cache_backprop(ctx, pos, nrm, target, weight, n, true, ctx->st)) return rc;
+    CK(cudaMemcpyAsync(ctx->hgrad ? ctx->hgrad : out_grad_host, ctx->cache_grad.p, (size_t)PM_CACHE_PARAMS * 4,
+                       cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemsetAsync(ctx->cache_grad.p, 0, (size_t)PM_CACHE_PARAMS * 4, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-    return check_status(ctx, "cache gradient");
+    const int rc = check_status(ctx, "cache gradient");
+    if (ctx->hgrad) std::memcpy(out_grad_host, ctx->hgrad, (size_t)PM_CACHE_PARAMS * 4);
+    if (out_loss) *out_loss = cache_loss_of(ctx, n);
+    return rc;
 }
 
 int pm_cache_infer(pm_ctx* ctx, const float* pos, const float* nrm, int64_t n, float* out_rgb) {

@@ -45,8 +45,9 @@ struct pm_ctx {
     bool own_stream = false;
     // pinned host words the small per-call device reads land in (a read into
     // pageable memory is staged by the driver): [0] status, [2..3] photon
-    // totals, [4..5] grid count maxima, [6..7] request count
+    // totals, [4] loss sum, [6..7] request count, [8..11] grid counts
     uint32_t* hbuf = nullptr;
+    float* hgrad = nullptr;    // page-locked copy of a gradient call's result (first call on)
     std::string err;
     int sm_count = 148;
     int trace_refill = 0;      // k_trace refill threshold; 0: the kernel's default
@@ -69,7 +70,7 @@ struct pm_ctx {
     pm::DevBuf status, gws;
     // learned radiance cache
     bool has_cache = false;
-    pm::DevBuf cache_w32, cache_w16, cache_m, cache_v, cache_grad, cache_loss;
+    pm::DevBuf cache_w32, cache_w16, cache_m, cache_v, cache_grad;   // cache_grad: the loss sum behind it
     // BVH: builder for the next pm_set_scene; the current scene's builder, size, build time
     int bvh_builder = 0, scene_bvh_builder = 0;
     int64_t bvh_nodes = 0;

@@ -90,7 +90,7 @@ Requests requests_of(pm_learned_graph* g) {
 uint64_t read_set(pm_ctx* ctx) {
     std::vector<DevBuf*> v = {&ctx->tri, &ctx->tri_pos, &ctx->tri_nrm, &ctx->tri_diffuse, &ctx->nodes, &ctx->prim,
                               &ctx->maabb, &ctx->mats, &ctx->ca, &ctx->tri_leaf, &ctx->status, &ctx->cache_w32,
-                              &ctx->cache_w16, &ctx->cache_m, &ctx->cache_v, &ctx->cache_grad, &ctx->cache_loss};
+                              &ctx->cache_w16, &ctx->cache_m, &ctx->cache_v, &ctx->cache_grad};
     for (auto& m : ctx->maps)
         for (DevBuf* b : {&m.pos, &m.dir, &m.pow, &m.starts, &m.sizes, &m.gpos, &m.gdir, &m.gpow, &m.cid, &m.keys0,
                           &m.keys1, &m.vals0, &m.vals1, &m.hist, &m.scan_ws, &m.small, &m.key_counts,
@@ -138,8 +138,7 @@ int enqueue_frame(pm_learned_graph* g) {
     if (g->steps > 0) {
         // the gradient starts at zero (each Adam step zeroes it after use); the
         // loss is not read back by a replayed frame
-        CK(cudaMemsetAsync(ctx->cache_grad.p, 0, (size_t)PM_CACHE_PARAMS * 4, st));
-        CK(cudaMemsetAsync(ctx->cache_loss.p, 0, 4, st));
+        CK(cudaMemsetAsync(ctx->cache_grad.p, 0, (size_t)(PM_CACHE_PARAMS + 1) * 4, st));
     }
     for (int s = 0; s < g->steps; s++) {
         MlpInputs in{};
@@ -149,7 +148,7 @@ int enqueue_frame(pm_learned_graph* g) {
         in.base_dev = state_offset(g);
         in.base_wrap = g->pool_n;
         CK(mlp_train(net, in, g->pool_target, nullptr, 2.f / (3.f * (float)g->batch), P<float>(ctx->cache_grad),
-                     P<float>(ctx->cache_loss), status, ctx->sm_count, st));
+                     P<float>(ctx->cache_grad) + PM_CACHE_PARAMS, status, ctx->sm_count, st));
         k_pool_step<<<1, 1, 0, st>>>(state_offset(g), g->pool_n, g->batch, state_step(g));
         CK(cudaGetLastError());
         CK(mlp_adam_dev(P<float>(ctx->cache_w32), P<__nv_bfloat16>(ctx->cache_w16), P<float>(ctx->cache_grad),
