@@ -1393,7 +1393,7 @@ int render_finish(pm_ctx* ctx, const pm_render_opts* o, FrameSetup& F, uint8_t* 
 
 namespace {
 
-// The gather visits the requests in Morton order of their hit points: 27-bit
+// The gather visits the requests in Morton order of their hit points: 18-bit
 // keys in the scene box, sorted by the library's stable radix sort on stream st.
 int request_order(pm_ctx* ctx, FrameSetup& F, cudaStream_t st) {
     F.ordered = true;
