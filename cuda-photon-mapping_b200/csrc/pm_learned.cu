@@ -15,29 +15,31 @@ namespace pm {
 
 namespace {
 
-// probe position k of P inside a tile of edge T: a ceil(sqrt(P)) grid of cell centres
-// Each probe's request: the first request of its pixel, which the probe pass
-// (probe_hits) traced from the camera with the eye pass's own device code;
-// the two records must agree bit for bit, and a probe whose record differs
-// from its request raises ST_BAD_INPUT (its request index is then dropped).
+// the request of probe s (its pixel's first request when that needs the global
+// estimate), else UINT32_MAX; s = tile * P + lattice point
+__device__ __forceinline__ uint32_t probe_request(const CameraDev& cam, const Requests& R, int tile, int P, int tiles_x,
+                                                  int64_t s) {
+    const int64_t t = s / P;
+    int dx, dy;
+    probe_xy((int)(s % P), P, tile, dx, dy);
+    const int x = (int)(t % tiles_x) * tile + dx, y = (int)(t / tiles_x) * tile + dy;
+    if (x >= cam.W || y >= cam.H) return 0xffffffffu;
+    const int64_t px = (int64_t)y * cam.W + x;
+    if (R.px_count[px] == 0) return 0xffffffffu;
+    const uint32_t r = R.px_base[px];
+    return (__float_as_uint(R.b[r].w) & 1u) ? r : 0xffffffffu;
+}
+
+// Each probe's request beside the record that the probe pass (probe_hits)
+// traced from the camera with the eye pass's own device code; the two must
+// agree bit for bit, and a probe whose record differs from its request raises
+// ST_BAD_INPUT (its request index is then dropped).
 __global__ void k_probe_req(CameraDev cam, Requests R, int tile, int P, int tiles_x, int64_t ntiles,
                             const float4* __restrict__ ppos, const float4* __restrict__ pnrm,
                             uint32_t* __restrict__ preq, unsigned* status) {
     const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= ntiles * P) return;
-    const int64_t t = s / P;
-    const int k = (int)(s % P);
-    int dx, dy;
-    probe_xy(k, P, tile, dx, dy);
-    const int x = (int)(t % tiles_x) * tile + dx, y = (int)(t / tiles_x) * tile + dy;
-    uint32_t q = 0xffffffffu;
-    if (x < cam.W && y < cam.H) {
-        const int64_t px = (int64_t)y * cam.W + x;
-        if (R.px_count[px] > 0) {
-            const uint32_t r = R.px_base[px];
-            if (__float_as_uint(R.b[r].w) & 1u) q = r;
-        }
-    }
+    uint32_t q = probe_request(cam, R, tile, P, tiles_x, s);
     const float4 pa = ppos[s], pb = pnrm[s];
     const bool probe = (__float_as_uint(pb.w) & 1u) != 0u;
     bool same = probe == (q != 0xffffffffu);
@@ -52,6 +54,25 @@ __global__ void k_probe_req(CameraDev cam, Requests R, int tile, int P, int tile
         raise_status(status, ST_BAD_INPUT);
         q = 0xffffffffu;
     }
+    preq[s] = q;
+}
+
+// After an eye pass on the same stream the probes' records are its requests:
+// this reads them (5 us at 1080p) where probe_hits would trace those pixels a
+// second time (0.17 ms, the latency of the longest of its rays).
+__global__ void k_probe_take(CameraDev cam, Requests R, int tile, int P, int tiles_x, int64_t ntiles,
+                             float4* __restrict__ ppos, float4* __restrict__ pnrm, uint32_t* __restrict__ preq) {
+    const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= ntiles * P) return;
+    const uint32_t q = probe_request(cam, R, tile, P, tiles_x, s);
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = make_float4(0.f, 0.f, 1.f, 0.f);
+    if (q != 0xffffffffu) {
+        a = R.a[q];
+        b = R.b[q];
+        b.w = __uint_as_float(1u);
+    }
+    ppos[s] = a;
+    pnrm[s] = b;
     preq[s] = q;
 }
 
@@ -160,6 +181,14 @@ cudaError_t learned_probe_req(const CameraDev& cam, const Requests& R, int tile,
     const int tx = (cam.W + tile - 1) / tile, ty = (cam.H + tile - 1) / tile;
     const int64_t ntiles = (int64_t)tx * ty;
     k_probe_req<<<blocks(ntiles * P, 256), 256, 0, st>>>(cam, R, tile, P, tx, ntiles, ppos, pnrm, preq, status);
+    return cudaGetLastError();
+}
+
+cudaError_t learned_probe_take(const CameraDev& cam, const Requests& R, int tile, int P, float4* ppos, float4* pnrm,
+                               uint32_t* preq, cudaStream_t st) {
+    const int tx = (cam.W + tile - 1) / tile, ty = (cam.H + tile - 1) / tile;
+    const int64_t ntiles = (int64_t)tx * ty;
+    k_probe_take<<<blocks(ntiles * P, 256), 256, 0, st>>>(cam, R, tile, P, tx, ntiles, ppos, pnrm, preq);
     return cudaGetLastError();
 }
 

@@ -16,6 +16,11 @@ constexpr uint32_t LEARNED_FALLBACK = 4u;   // request flag: answered by the exa
 cudaError_t learned_probe_req(const CameraDev& cam, const Requests& R, int tile, int P, const float4* ppos,
                               const float4* pnrm, uint32_t* preq, unsigned* status, cudaStream_t st);
 
+// The probes' records (those of probe_hits) and requests read from the eye
+// pass's requests: a pixel's first request is its primary hit.
+cudaError_t learned_probe_take(const CameraDev& cam, const Requests& R, int tile, int P, float4* ppos, float4* pnrm,
+                               uint32_t* preq, cudaStream_t st);
+
 // Tile flags from the probes' exact and cached estimates (bias above
 // max_rel_err plus noise_z standard errors), then flag bit
 // LEARNED_FALLBACK on every global request of a flagged tile, whose index also
