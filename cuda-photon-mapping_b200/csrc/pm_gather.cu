@@ -74,6 +74,7 @@ struct Staged {
     float block2;             // squared distance to the nearest face of the 27 sub-cells with sub-cells behind it
     float bscale;             // NB / lim2
 };
+constexpr float BLOCK_MARGIN = 1.f + 2e-5f;   // of squared bounds over box distances: above their rounding
 enum { Q_ACTIVE = 1, Q_GUESSED = 2, Q_WIDE = 4 };
 
 // Shared memory of a block of NW warps: its queries and each warp's store.
@@ -344,8 +345,11 @@ __device__ __forceinline__ Cube cube_of(const GatherGrid& G, const GatherReach& 
                 min(G.gy - 1, cy + E.rc), min(G.gz - 1, cz + E.rc)};
 }
 
-// The set-up of one query by one thread (by the query's own warp it took a fifth
-// of the query's instructions).
+// The set-up of one query: by one thread (by the query's own warp it took a fifth
+// of the query's instructions), or, WARP, by all lanes of a warp where a block
+// has no more queries than warps and only the latency counts (one thread's nine
+// dependent rows take 9,500 cycles, more than the rest of a query that finds few
+// photons).
 //
 // Density guess of the bound on the k-th distance: the N photons of the 27
 // sub-cells around the query, spread over a plane through them (area 9 sc^2),
@@ -354,6 +358,7 @@ __device__ __forceinline__ Cube cube_of(const GatherGrid& G, const GatherReach& 
 // padded box lies farther than g is not scanned at all; when fewer than k
 // photons lie within g, the query starts again with the bound r, so the answer
 // is unchanged.
+template <bool WARP = false>
 __device__ __forceinline__ void stage_query(const GatherGrid& G, const GatherReach& E, Staged& s, V3 q, int k,
                                             int flags) {
     int cx, cy, cz, sx, sy, sz;
@@ -369,32 +374,23 @@ __device__ __forceinline__ void stage_query(const GatherGrid& G, const GatherRea
     uint32_t N = 0u;
     const int xl = max(X0 - 1, lx), xr = min(X0 + 1, hx);
     const bool cut = S > 1 && (xl >> sh) != (xr >> sh);   // the row crosses into the next cell
+    auto row = [&](int dy, int dz) -> uint32_t {   // photons of three sub-cells along x
+        const int Y = Y0 + dy, Z = Z0 + dz;
+        if (xl > xr || Y < ly || Y > hy || Z < lz || Z > hz) return 0u;
+        if (!cut) return __ldg(G.key_starts + sub_key(G, xr, Y, Z, sh) + 1) - __ldg(G.key_starts + sub_key(G, xl, Y, Z, sh));
+        const int xm = (xr >> sh) << sh;
+        return __ldg(G.key_starts + sub_key(G, xm - 1, Y, Z, sh) + 1) - __ldg(G.key_starts + sub_key(G, xl, Y, Z, sh)) +
+               __ldg(G.key_starts + sub_key(G, xr, Y, Z, sh) + 1) - __ldg(G.key_starts + sub_key(G, xm, Y, Z, sh));
+    };
+    if (WARP) {
+        const int lane = threadIdx.x & 31;
+        N = __reduce_add_sync(0xffffffffu, lane < 9 ? row(lane % 3 - 1, lane / 3 - 1) : 0u);
+        if (lane != 0) return;
+    } else {
 #pragma unroll 1
-    for (int dz = -1; dz <= 1; dz++)
+        for (int dz = -1; dz <= 1; dz++)
 #pragma unroll
-        for (int dy = -1; dy <= 1; dy++) {
-            const int Y = Y0 + dy, Z = Z0 + dz;
-            if (xl > xr || Y < ly || Y > hy || Z < lz || Z > hz) continue;
-            if (!cut) {
-                N += __ldg(G.key_starts + sub_key(G, xr, Y, Z, sh) + 1) - __ldg(G.key_starts + sub_key(G, xl, Y, Z, sh));
-            } else {
-                const int xm = (xr >> sh) << sh;
-                N += __ldg(G.key_starts + sub_key(G, xm - 1, Y, Z, sh) + 1) - __ldg(G.key_starts + sub_key(G, xl, Y, Z, sh));
-                N += __ldg(G.key_starts + sub_key(G, xr, Y, Z, sh) + 1) - __ldg(G.key_starts + sub_key(G, xm, Y, Z, sh));
-            }
-        }
-    s.lim2 = r2;
-    if (G.guess > 0.f && N > (uint32_t)k) {   // else too few photons in the block to gain anything
-        const float g2 = 9.f * sc * sc * (G.guess * (float)k) / (3.14159265f * (float)N);
-        if (g2 < r2) {
-            s.lim2 = g2;
-            flags |= Q_GUESSED;
-        }
-    } else if (N < (uint32_t)k) {
-        // fewer than k in the block: the sphere of the guess, beyond the block
-        const float per = G.guess > 0.f ? G.guess : GATHER_GUESS;
-        s.lim2 = fminf(r2, N > 0u ? 9.f * sc * sc * (per * (float)k) / (3.14159265f * (float)N) : 64.f * sc * sc);
-        flags |= Q_WIDE;
+            for (int dy = -1; dy <= 1; dy++) N += row(dy, dz);
     }
     auto face = [&](float p, float mn, int X, int lo, int hi) {
         const float a = X - 1 > lo ? p - (mn + (X - 1) * sc) : INFINITY, b = X + 1 < hi ? mn + (X + 2) * sc - p : INFINITY;
@@ -402,7 +398,27 @@ __device__ __forceinline__ void stage_query(const GatherGrid& G, const GatherRea
     };
     const float f = fminf(fminf(face(q.x, G.mn[0], X0, lx, hx), face(q.y, G.mn[1], Y0, ly, hy)),
                           face(q.z, G.mn[2], Z0, lz, hz)) - E.pad;
-    s.block2 = f > 0.f ? f * f : 0.f;
+    const float block2 = f > 0.f ? f * f : 0.f;
+    s.block2 = block2;
+    s.lim2 = r2;
+    if (G.guess > 0.f && N > (uint32_t)k) {   // else too few photons in the block to gain anything
+        const float g2 = 9.f * sc * sc * (G.guess * (float)k) / (3.14159265f * (float)N);
+        if (g2 < r2) {
+            s.lim2 = g2;
+            flags |= Q_GUESSED;
+        }
+    } else if (N < (uint32_t)k && !(r2 * BLOCK_MARGIN < block2)) {
+        // fewer than k in the block and more of r's sphere beyond it: the
+        // sphere of the guess (at once that of r where it hardly leaves the
+        // block).  Where none of r's sphere lies beyond, the 27 sub-cells in the
+        // walk's own order, bound r, answer the query: as a growing sphere, its
+        // answer ordered afterwards, 61,779 requests of the small room (k 100)
+        // took 0.174 ms instead of 0.143.
+        const float per = G.guess > 0.f ? G.guess : GATHER_GUESS;
+        if (r2 > 4.f * sc * sc)
+            s.lim2 = fminf(r2, N > 0u ? 9.f * sc * sc * (per * (float)k) / (3.14159265f * (float)N) : 64.f * sc * sc);
+        flags |= Q_WIDE;
+    }
     s.qx = q.x; s.qy = q.y; s.qz = q.z;
     s.X0 = X0; s.Y0 = Y0; s.Z0 = Z0;
     s.flags = flags;
@@ -492,6 +508,17 @@ __device__ __forceinline__ void shells_order(const GatherGrid& G, const GatherRe
         if (wide) {
             warp_sort_keys(key, cnt, lane);
         } else if (__all_sync(0xffffffffu, fits)) {
+            if (cnt <= 32) {   // one key per lane: its rank by comparing it with the others
+                const uint32_t v = lane < cnt ? key32[lane] : 0u;
+                const uint2 x = U.ent[lane];
+                int rank = 0;
+#pragma unroll 1
+                for (int e = 0; e < cnt; e++) rank += (int)(__shfl_sync(0xffffffffu, v, e) < v);
+                __syncwarp();
+                if (lane < cnt) out[rank] = x;
+                __syncwarp();
+                return;
+            }
             if (cnt <= 64) sort_u32<2>(key32, cnt, lane);
             else if (cnt <= 128) sort_u32<4>(key32, cnt, lane);
             else sort_u32<8>(key32, cnt, lane);
@@ -507,6 +534,67 @@ __device__ __forceinline__ void shells_order(const GatherGrid& G, const GatherRe
 #pragma unroll
     for (int r = 0; r < 8; r++)
         if (32 * r + lane < cnt) out[32 * r + lane] = v[r];
+    __syncwarp();
+}
+
+// The ids of the answer's entries (cnt <= k <= UCAP / 2, in one half of the store)
+// by ascending (distance, id).  The entries are put into NB bins of equal width
+// over [0, rk] in the other half (the bin of a distance grows with it, and equal
+// distances share one); an entry's place is its bin's first one plus the entries
+// of its bin that come before it.  A bitonic sort of the 64-bit keys in shared
+// memory took 36 passes at k 200 (photons set, grid, 100,003 queries with ids
+// at k 200: 2.15 ms, now 1.77).
+template <int UCAP>
+__device__ __noinline__ void write_ids(WarpStore<UCAP>& U, const float4* gpos, const uint2* ent, int cnt, int k, float rk,
+                                       uint32_t* ids, int lane) {
+    unsigned long long* key = reinterpret_cast<unsigned long long*>(U.ent);
+    unsigned long long* out = key;
+    (ent == U.ent ? out : key) += UCAP / 2;
+    const float scale = (float)NB / rk;   // (rk 0: all in bin 0 or NB - 1 alike)
+    auto bin = [&](unsigned long long x) {
+        return min((int)(__uint_as_float((uint32_t)(x >> 32)) * scale), NB - 1);
+    };
+    __syncwarp();
+    reinterpret_cast<uint2*>(U.dh)[lane] = make_uint2(0u, 0u);
+    __syncwarp();
+#pragma unroll 1
+    for (int e = lane; e < cnt; e += 32) {
+        const uint2 x = ent[e];
+        const unsigned long long v = (unsigned long long)__float_as_uint(sqrtf(__uint_as_float(x.x))) << 32 |
+                                     __float_as_uint(__ldg(&gpos[x.y].w));
+        key[e] = v;
+        atomicAdd(&U.dh[bin(v)], 1u);
+    }
+    __syncwarp();
+    const uint2 c = reinterpret_cast<uint2*>(U.dh)[lane];
+    uint32_t incl = c.x + c.y;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    reinterpret_cast<uint2*>(U.dh)[lane] = make_uint2(incl - c.x - c.y, incl - c.y);
+    __syncwarp();
+#pragma unroll 1
+    for (int e = lane; e < cnt; e += 32) {
+        const unsigned long long v = key[e];
+        out[atomicAdd(&U.dh[bin(v)], 1u)] = v;   // dh: from a bin's first place to the next bin's
+    }
+    __syncwarp();
+#pragma unroll 1
+    for (int e = lane; e < k; e += 32) {
+        if (e >= cnt) {
+            ids[e] = 0xffffffffu;
+            continue;
+        }
+        const unsigned long long v = out[e];
+        const int b = bin(v);
+        const int lo = b > 0 ? (int)U.dh[b - 1] : 0, hi = (int)U.dh[b];
+        int place = lo;
+#pragma unroll 1
+        for (int q = lo; q < hi; q++) place += (int)(out[q] < v);
+        ids[place] = (uint32_t)v;
+    }
     __syncwarp();
 }
 
@@ -535,7 +623,7 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
     int mode = s.flags & Q_WIDE ? M_WIDE : M_RING, base = 0, total = 27;
     bool coarse = false;       // M_WIDE: rows of cells, not of sub-cells
     bool plan = mode == M_WIDE;   // the box of rows is still to be set
-    const float m2 = 1.f + 2e-5f;
+    const float m2 = BLOCK_MARGIN;
     reinterpret_cast<uint2*>(U.dh)[lane] = make_uint2(0u, 0u);
     __syncwarp();
     coarse = plan && lim2 > 16.f * E.sc * E.sc && E.sh > 0;
@@ -723,7 +811,7 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
             continue;
         }
         if (lim2 == E.r2) {           // all within r is found ...
-            if (mode == M_WIDE || s.block2 == INFINITY) break;
+            if (mode == M_WIDE || lim2 * m2 < s.block2) break;
             mode = M_WIDE;            // ... in the 27 sub-cells: with the guess that they give, or r
             lim2 = fminf(E.r2, 9.f * E.sc * E.sc * GATHER_GUESS * __fdividef((float)k, 3.14159265f * (float)max(n, 1)));
         } else if (mode == M_WIDE) {  // the sphere held too few: a larger one
@@ -821,19 +909,7 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
         if (O.rk) O.rk[i] = rk;
     }
     if (O.ids) {
-        // ascending (distance, id)
-        unsigned long long* key = reinterpret_cast<unsigned long long*>(ent);
-#pragma unroll 1
-        for (int e = lane; e < cnt; e += 32) {
-            const uint2 x = ent[e];
-            key[e] = (unsigned long long)__float_as_uint(sqrtf(__uint_as_float(x.x))) << 32 |
-                     __float_as_uint(__ldg(&G.gpos[x.y].w));
-        }
-        __syncwarp();
-        warp_sort_keys(key, cnt, lane);
-#pragma unroll 1
-        for (int e = lane; e < k; e += 32)
-            O.ids[i * k + e] = e < cnt ? (uint32_t)(key[e] & 0xffffffffull) : 0xffffffffu;
+        write_ids<UCAP>(U, G.gpos, ent, cnt, k, rk, O.ids + i * k, lane);
     }
     __syncwarp();
 }
@@ -866,14 +942,16 @@ __device__ __forceinline__ const float* normal_of(const GatherQueries& Q, int64_
 }
 
 // Queries 0 .. cnt - 1 of a block (cnt <= its threads).  Each thread sets one
-// query up, then the warps take them in order: neighbouring queries (the frame's
+// query up (FEW: each warp), then the warps take them in order: neighbouring queries (the frame's
 // come in Morton order) run at the same time on an SM and share its L1 (32
 // consecutive queries per warp instead: 0.5 ms more for the 10M-photon frame).
-template <int UCAP, int NW, class Stage, class Answer>
+// FEW: no more queries than warps.
+template <int UCAP, int NW, bool FEW = false, class Stage, class Answer>
 __device__ __forceinline__ void block_queries(BlockSmem<UCAP, NW>& M, int cnt, const Stage& stage, const Answer& answer) {
     const int lane = threadIdx.x & 31;
     if (threadIdx.x == 0) M.next = 0;
-    if ((int)threadIdx.x < cnt) stage((int)threadIdx.x);
+    const int own = FEW ? (int)threadIdx.x >> 5 : (int)threadIdx.x;
+    if (own < cnt) stage(own);
     __syncthreads();
 #pragma unroll 1
     while (true) {
@@ -885,18 +963,18 @@ __device__ __forceinline__ void block_queries(BlockSmem<UCAP, NW>& M, int cnt, c
     }
 }
 
-template <int UCAP>
+template <int UCAP, bool FEW = false>
 __device__ __forceinline__ void gather_block(const GatherGrid& G, const GatherReach& E, BlockSmem<UCAP, WARPS>& M,
                                              const GatherQueries& Q, int64_t q0, int cnt, int k, int require_full,
                                              const GatherOut& O, float inv_norm) {
     const int lane = threadIdx.x & 31;
     WarpStore<UCAP>& U = M.st[threadIdx.x >> 5];
-    block_queries(
+    block_queries<UCAP, WARPS, FEW>(
         M, cnt,
         [&](int t) {
             V3 q;
             const bool active = load_query(Q, record_of(Q, q0 + t), q) && k > 0;
-            if (active) stage_query(G, E, M.q[t], q, k, Q_ACTIVE);
+            if (active) stage_query<FEW>(G, E, M.q[t], q, k, Q_ACTIVE);
             else M.q[t].flags = 0;
         },
         [&](int t) {
@@ -908,13 +986,14 @@ __device__ __forceinline__ void gather_block(const GatherGrid& G, const GatherRe
         });
 }
 
-template <int UCAP>
+// FEW: launched with one query per warp (per == WARPS)
+template <int UCAP, bool FEW>
 __global__ void __launch_bounds__(WARPS * 32, 4)
 k_gather(GatherGrid G, GatherReach E, GatherQueries Q, int k, int require_full, GatherOut O, int per) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int64_t q0 = (int64_t)blockIdx.x * per;
-    gather_block<UCAP>(G, E, *reinterpret_cast<BlockSmem<UCAP, WARPS>*>(smem_raw), Q, q0,
-                       (int)min((int64_t)per, Q.n - q0), k, require_full, O, filter_norm());
+    gather_block<UCAP, FEW>(G, E, *reinterpret_cast<BlockSmem<UCAP, WARPS>*>(smem_raw), Q, q0,
+                            (int)min((int64_t)per, Q.n - q0), k, require_full, O, filter_norm());
 }
 
 // Queries a block takes at a time from n, for `blocks` resident ones: one per
@@ -1033,11 +1112,12 @@ template <int UCAP>
 cudaError_t launch(const GatherGrid& G, const GatherQueries& Q, float r, int k, int require_full, const GatherOut& O,
                    cudaStream_t st) {
     const size_t smem = sizeof(BlockSmem<UCAP, WARPS>);
-    cudaError_t e = cudaFuncSetAttribute(k_gather<UCAP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
     const int per = block_chunk(Q.n, 4 * 148, WARPS);
+    const auto kernel = per == WARPS ? k_gather<UCAP, true> : k_gather<UCAP, false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
     const unsigned blocks = (unsigned)((Q.n + per - 1) / per);
-    k_gather<UCAP><<<blocks, WARPS * 32, smem, st>>>(G, gather_reach(G, r), Q, k, require_full, O, per);
+    kernel<<<blocks, WARPS * 32, smem, st>>>(G, gather_reach(G, r), Q, k, require_full, O, per);
     return cudaGetLastError();
 }
 
