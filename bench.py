@@ -190,6 +190,12 @@ class ClockSampler:
 
 
 # ----------------------------------------------------------------- CPU leg
+def reference_missing():
+    """Why the reference's host library cannot be loaded here (None: it can)."""
+    lib = os.path.join(os.path.dirname(os.path.abspath(__file__)), "oracle", "_ref", "libref_host.so")
+    return None if os.path.exists(lib) else "oracle/_ref/libref_host.so was not built: the reference's sources are not here"
+
+
 def cpu_reference_estimate(sc, w, rows=8, trace_paths=16384, threads=None):
     """The reference's CPU path on the host cores, on a bounded sample, scaled
     to one full frame of the workload.
@@ -731,7 +737,7 @@ def run_ours(args):
                                                                                   or args.height)))
         dominant = max(kernels, key=lambda k: kernels[k]["ms_per_launch"])
         cpu = None
-        if not args.no_cpu_baseline:
+        if not args.no_cpu_baseline and reference_missing() is None:
             est = cpu_reference_estimate(sc, w)
             cpu = {"value": w["photons"] / est["step_s"] / 1e6, "unit": "Mphotons/s", "cores": est["cores"],
                    "kind": "reference", "sample": est["sample"],
@@ -773,6 +779,8 @@ def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return None
+    if reference_missing():
+        return {"impl": "reference", "unavailable": reference_missing()}
     sc, cs, w = scenes.workload(args.workload)
     ests = []
     for i in range(args.warmup + args.steps):
