@@ -570,7 +570,8 @@ def learned_rmse(ctx, sc, cs, cam, w):
 # default workload's two large kernels: constants from one ncu capture of the
 # timed step's launches (the line names the capture in "traffic_source")
 DRAM_TRAFFIC = {"k_trace": 149_363_200 + 429_206_272, "k_gather": 333_646_592 + 13_331_456}
-TRAFFIC_SOURCE = ("constant from one ncu capture of the default workload (the timed step's launches): ncu --metrics "
+TRAFFIC_SOURCE = ("constant from one ncu capture of the default workload on an earlier build (the timed step's launches): "
+                  "ncu --metrics "
                   "gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum --clock-control none "
                   "-c 400 python bench.py --steps 1 --warmup 1 --no-cpu-baseline --no-learned --no-batched")
 FP32_PEAK_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12   # 148 SMs x 128 FP32 lanes x 2 flop (FMA) x 1965 MHz
