@@ -790,7 +790,7 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
                 const float4 p = __ldg(G.gpos + j);
                 const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
                 const float d2 = dx * dx + dy * dy + dz * dz;
-                enter(p0 + lane < photons ? d2 : INFINITY, j);
+                enter(p0 + lane < photons ? d2 : __int_as_float(0x7fffffff), j);   // NaN is within no bound, infinity within that of r = inf
             }
         }
         qn = 0;
