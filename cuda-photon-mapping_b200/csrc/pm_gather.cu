@@ -45,6 +45,7 @@
 #include <type_traits>
 #include "pm_gather.cuh"
 #include "pm_device.cuh"
+#include "pm_div.h"
 
 namespace pm {
 
@@ -101,15 +102,6 @@ __device__ __forceinline__ float axis_gap(float q, float lo, float hi, bool open
     float a = open_lo ? 0.f : lo - q;
     float b = open_hi ? 0.f : q - hi;
     return fmax3(a, b, 0.f);
-}
-
-// u / d for 0 <= u < 2^22, d > 0: float estimate, one correction step
-__device__ __forceinline__ int small_div(int u, int d, float inv) {
-    int q = (int)(((float)u + 0.5f) * inv);
-    const int r = u - q * d;
-    if (r < 0) q--;
-    else if (r >= d) q++;
-    return q;
 }
 
 // Place of the sub-cell at offset (dx, dy, dz) in its shell at Chebyshev distance

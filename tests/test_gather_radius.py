@@ -37,3 +37,27 @@ def test_radius_beyond_the_map(sub_div, photons, radius):
         np.testing.assert_allclose(rad.cpu().numpy()[ok], ref[ok], rtol=1e-5)
     assert ctx.status() == 0
     ctx.close()
+
+
+@pytest.mark.gpu
+def test_box_of_ten_million_rows():
+    """A sphere that covers a grid of 3 x 400 x 400 cells, each cut 8 ways: 10.24M
+    rows of sub-cells in 3 runs each."""
+    import torch
+    import photonmap
+    rng = np.random.default_rng(2)
+    size = np.array([3, 400, 400], np.float32)
+    pos = (rng.random((480_000, 3)) * size).astype(np.float32)
+    pos[-3:] = size - np.float32(0.01)      # the last sub-cell of the last row holds photons
+    ctx = photonmap.Context(0)
+    ctx.set_photons(0, pos, np.ones_like(pos), np.ones_like(pos))
+    ctx.build_grid(0, aabb=np.concatenate([0 * size, size]), sub_div=8, desired=1)
+    assert ctx.photons(0)["dims"] == (3, 400, 400)
+    q = np.array([[-2000, 200, 200], [1.5, 200, 3000], [1.5, 900, 900]], np.float32)
+    qn = np.zeros_like(q)
+    for k in (8, 256):
+        _, ids, cnt = ctx.gather(torch.from_numpy(q), torch.from_numpy(qn), k, 1e4, want_ids=True)
+        want, _ = _exhaustive(pos, np.ones_like(pos), np.ones_like(pos), q, qn, k, 1e4)
+        assert np.array_equal(ids.cpu().numpy(), want), k
+    assert ctx.status() == 0
+    ctx.close()
