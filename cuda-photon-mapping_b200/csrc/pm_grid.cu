@@ -467,6 +467,7 @@ k_radix_pass(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ 
             // (the whole warp: a shuffle per group of equal digits runs the groups one after another)
             old = __shfl_sync(0xffffffffu, old, leader);
             r[j] = old + (uint32_t)__popc(peers & lanemask_lt());
+            __syncwarp();   // the next step's leader of a digit may be another lane: it reads this step's count
         }
         __syncthreads();
         // exclusive prefix of each digit over warps; the tile's count

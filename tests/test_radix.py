@@ -41,3 +41,27 @@ def test_grid_order_is_a_stable_sort(n, spread):
     assert torch.equal(g["cell_sizes"].long(), counts)
     assert torch.equal(g["cell_starts"].long(), torch.cumsum(counts, 0) - counts)
     ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("m", [1, 2, 3, 31, 32, 33])
+@pytest.mark.parametrize("n", [512 * 9 - 5, 512 * 3600 - 13])        # look-back, runs
+def test_running_counts_pass_from_lane_to_lane(n, m):
+    """Keys whose leader lane moves from one step of 32 to the next, so that each
+    step reads the running count that another lane wrote."""
+    import torch
+    import photonmap
+    i = torch.arange(n, device="cuda")
+    lane, step = i & 31, i >> 5
+    key = (lane + step) % m                                 # m sub-cells along x, rotated by one lane a step
+    pos = torch.zeros((n, 3), device="cuda")
+    pos[:, 0] = (key.float() + 0.5) / 64
+    pw = torch.full_like(pos, 0.5)
+    ctx = photonmap.Context(0)
+    ctx.set_photons(0, pos, pw, pw)
+    ctx.build_grid(0, aabb=BOX, sub_div=8, desired=-(-n // 512), regrid_mult=1000)   # 64 sub-cells along x
+    g = ctx.photons(0)
+    assert g["dims"] == (8, 8, 8) and g["cell"] == 0.125
+    order = g["sorted_pos"][:, 3].contiguous().view(torch.int32).long()
+    assert torch.equal(order, torch.sort(key, stable=True).indices)
+    ctx.close()
