@@ -328,6 +328,19 @@ __device__ __noinline__ float overflow(WarpStore<UCAP>& U, const float4* gpos, i
     return d * d * 1.000001f;
 }
 
+// The largest float with the rounded root of s (at most three steps).  A first
+// bound is raised to it: distances are compared as rounded roots, so of photons
+// that share one either all are within the bound or none.
+__device__ __forceinline__ float same_root(float s) {
+    const float d = sqrtf(s);
+#pragma unroll 1
+    while (true) {
+        const float t = __uint_as_float(__float_as_uint(s) + 1u);
+        if (sqrtf(t) != d) return s;
+        s = t;
+    }
+}
+
 // the cells of the reference's cube around cell (cx, cy, cz)
 struct Cube {
     int x0, y0, z0, x1, y1, z1;
@@ -394,7 +407,7 @@ __device__ __forceinline__ void stage_query(const GatherGrid& G, const GatherRea
     s.block2 = block2;
     s.lim2 = r2;
     if (G.guess > 0.f && N > (uint32_t)k) {   // else too few photons in the block to gain anything
-        const float g2 = 9.f * sc * sc * (G.guess * (float)k) / (3.14159265f * (float)N);
+        const float g2 = same_root(9.f * sc * sc * (G.guess * (float)k) / (3.14159265f * (float)N));
         if (g2 < r2) {
             s.lim2 = g2;
             flags |= Q_GUESSED;
@@ -408,7 +421,7 @@ __device__ __forceinline__ void stage_query(const GatherGrid& G, const GatherRea
         // took 0.174 ms instead of 0.143.
         const float per = G.guess > 0.f ? G.guess : GATHER_GUESS;
         if (r2 > 4.f * sc * sc)
-            s.lim2 = fminf(r2, N > 0u ? 9.f * sc * sc * (per * (float)k) / (3.14159265f * (float)N) : 64.f * sc * sc);
+            s.lim2 = fminf(r2, same_root(N > 0u ? 9.f * sc * sc * (per * (float)k) / (3.14159265f * (float)N) : 64.f * sc * sc));
         flags |= Q_WIDE;
     }
     s.qx = q.x; s.qy = q.y; s.qz = q.z;
@@ -805,13 +818,14 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
         if (lim2 == E.r2) {           // all within r is found ...
             if (mode == M_WIDE || lim2 * m2 < s.block2) break;
             mode = M_WIDE;            // ... in the 27 sub-cells: with the guess that they give, or r
-            lim2 = fminf(E.r2, 9.f * E.sc * E.sc * GATHER_GUESS * __fdividef((float)k, 3.14159265f * (float)max(n, 1)));
+            lim2 = 9.f * E.sc * E.sc * GATHER_GUESS * __fdividef((float)k, 3.14159265f * (float)max(n, 1));
         } else if (mode == M_WIDE) {  // the sphere held too few: a larger one
-            lim2 = fminf(E.r2, lim2 * fmaxf(2.f, 1.5f * GATHER_GUESS * __fdividef((float)k, (float)max(n, 1))));
+            lim2 = lim2 * fmaxf(2.f, 1.5f * GATHER_GUESS * __fdividef((float)k, (float)max(n, 1)));
         } else {                      // the guess held too few of the 27: all of theirs within r
             lim2 = E.r2;
             plan = false;
         }
+        lim2 = fminf(E.r2, same_root(lim2));
         coarse = plan && lim2 > 16.f * E.sc * E.sc && E.sh > 0;
         bscale = lim2 == E.r2 ? E.bscale : __fdividef((float)NB, lim2);
         n = 0;

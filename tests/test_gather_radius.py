@@ -61,3 +61,51 @@ def test_box_of_ten_million_rows():
         assert np.array_equal(ids.cpu().numpy(), want), k
     assert ctx.status() == 0
     ctx.close()
+
+
+def _tied(target):
+    """(x, y) with x * x + y * y == target in float32."""
+    for x in np.linspace(0.6, 0.9, 4001, dtype=np.float32) * np.sqrt(target):
+        y = np.sqrt(target - x * x)
+        for _ in range(8):
+            y = np.nextafter(y, np.float32(0))
+        for _ in range(16):
+            if np.float32(x * x) + np.float32(y * y) == target:
+                return x, y
+            y = np.nextafter(y, np.float32(1))
+    raise AssertionError("no such point")
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("first", ["sphere", "guess"])
+def test_equal_distances_on_either_side_of_the_first_bound(first):
+    """The two farthest of k + 1 photons have one rounded distance, their squares
+    lie on either side of the walk's first bound: the smaller index stays."""
+    import torch
+    import photonmap
+    if first == "sphere":        # nothing in the 27 sub-cells of edge 1 / 8: (8 / 8)^2
+        k, S, lo, bound = 4, 8, 0.0, np.float32(1)
+        near = 0.5 * np.eye(3)
+        far = np.zeros((0, 3))
+    else:                        # the density guess of 1.6 k photons among N in a plane of 9 sub-cells of edge 1 / 4
+        k, S, lo = 8, 4, -0.5
+        for N in range(30, 60):
+            bound = np.float32(0.5625) * (np.float32(1.6) * np.float32(k)) / (np.float32(3.14159265) * np.float32(N))
+            if np.sqrt(bound) == np.sqrt(np.nextafter(bound, np.float32(1))):
+                break
+        near = np.stack([np.linspace(0.01, 0.1, k - 1), np.zeros(k - 1), np.zeros(k - 1)], 1)
+        far = np.stack([np.linspace(0.4, 0.45, N - k - 1), np.zeros(N - k - 1), np.zeros(N - k - 1)], 1)
+    beyond = np.nextafter(bound, np.float32(2))
+    assert np.sqrt(beyond) == np.sqrt(bound)
+    inside, outside = _tied(bound), _tied(beyond)
+    pos = np.concatenate([[[outside[0], outside[1], 0]], near, far, [[inside[0], inside[1], 0]]]).astype(np.float32)
+    one = np.ones_like(pos)
+    ctx = photonmap.Context(0)
+    ctx.set_photons(0, pos, one, one)
+    ctx.build_grid(0, aabb=np.array([lo] * 3 + [lo + 1] * 3, np.float32), sub_div=S, desired=1000)
+    q = np.zeros((1, 3), np.float32)
+    _, ids, _ = ctx.gather(torch.from_numpy(q), torch.from_numpy(q), k, 2.0, want_ids=True)
+    want, _ = _exhaustive(pos, one, one, q, q, k, 2.0)
+    assert 0 in want and len(pos) - 1 not in want
+    assert np.array_equal(ids.cpu().numpy(), want)
+    ctx.close()
