@@ -328,17 +328,16 @@ __device__ __noinline__ float overflow(WarpStore<UCAP>& U, const float4* gpos, i
     return d * d * 1.000001f;
 }
 
-// The largest float with the rounded root of s (at most three steps).  A first
-// bound is raised to it: distances are compared as rounded roots, so of photons
-// that share one either all are within the bound or none.
-__device__ __forceinline__ float same_root(float s) {
-    const float d = sqrtf(s);
-#pragma unroll 1
-    while (true) {
-        const float t = __uint_as_float(__float_as_uint(s) + 1u);
-        if (sqrtf(t) != d) return s;
-        s = t;
-    }
+// A first bound on squared distances, x raised by at most a thousandth so that it
+// is the largest square with its rounded root: distances are compared as
+// rounded roots, and of photons that share one either all are within the bound
+// or none.  The root d has 12 bits, so d * d is exact, and the squares beyond it
+// that round to d end before d * d + d ulp(d): at the next float where d's
+// mantissa is below sqrt(2) (an even exponent of d * d), at d * d itself elsewhere.
+__device__ __forceinline__ float tie_bound(float x) {
+    const float d = __uint_as_float((__float_as_uint(sqrt_approx(x)) + 0xfffu) & ~0xfffu);
+    const uint32_t s = __float_as_uint(d * d);
+    return __uint_as_float(s + (s >> 23 & 1u));   // (beyond the largest float: NaN, which fminf drops)
 }
 
 // the cells of the reference's cube around cell (cx, cy, cz)
@@ -407,7 +406,7 @@ __device__ __forceinline__ void stage_query(const GatherGrid& G, const GatherRea
     s.block2 = block2;
     s.lim2 = r2;
     if (G.guess > 0.f && N > (uint32_t)k) {   // else too few photons in the block to gain anything
-        const float g2 = same_root(9.f * sc * sc * (G.guess * (float)k) / (3.14159265f * (float)N));
+        const float g2 = tie_bound(9.f * sc * sc * (G.guess * (float)k) / (3.14159265f * (float)N));
         if (g2 < r2) {
             s.lim2 = g2;
             flags |= Q_GUESSED;
@@ -421,7 +420,7 @@ __device__ __forceinline__ void stage_query(const GatherGrid& G, const GatherRea
         // took 0.174 ms instead of 0.143.
         const float per = G.guess > 0.f ? G.guess : GATHER_GUESS;
         if (r2 > 4.f * sc * sc)
-            s.lim2 = fminf(r2, same_root(N > 0u ? 9.f * sc * sc * (per * (float)k) / (3.14159265f * (float)N) : 64.f * sc * sc));
+            s.lim2 = fminf(r2, tie_bound(N > 0u ? 9.f * sc * sc * (per * (float)k) / (3.14159265f * (float)N) : 64.f * sc * sc));
         flags |= Q_WIDE;
     }
     s.qx = q.x; s.qy = q.y; s.qz = q.z;
@@ -825,7 +824,7 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
             lim2 = E.r2;
             plan = false;
         }
-        lim2 = fminf(E.r2, same_root(lim2));
+        lim2 = lim2 < E.r2 ? fminf(E.r2, tie_bound(lim2)) : E.r2;
         coarse = plan && lim2 > 16.f * E.sc * E.sc && E.sh > 0;
         bscale = lim2 == E.r2 ? E.bscale : __fdividef((float)NB, lim2);
         n = 0;
