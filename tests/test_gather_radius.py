@@ -109,3 +109,51 @@ def test_equal_distances_on_either_side_of_the_first_bound(first):
     assert 0 in want and len(pos) - 1 not in want
     assert np.array_equal(ids.cpu().numpy(), want)
     ctx.close()
+
+
+def _time(ctx, q, qn, k, radius):
+    import torch
+    best = float("inf")
+    for _ in range(6):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda.synchronize()
+        a.record()
+        ctx.gather(q, qn, k, radius)
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b))
+    return best
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [16, 200])
+def test_time_does_not_grow_with_a_radius_that_holds_more_than_k(k):
+    """Photons on the walls of a box and on a ball that lies on its floor; the radius
+    stops mattering once it holds k photons.  Near the ball the density guess
+    holds too few (such walks, their next bound the radius itself, made the calls
+    take several times as long with a radius of 100 boxes)."""
+    import torch
+    import photonmap
+    gen = torch.Generator(device="cuda")
+    gen.manual_seed(4)
+
+    def photons(n):
+        p = torch.rand((n, 3), generator=gen, device="cuda") * 2 - 1
+        axis = torch.randint(0, 3, (n, 1), generator=gen, device="cuda")
+        p = p.scatter(1, axis, torch.where(torch.rand((n, 1), generator=gen, device="cuda") < 0.5, -1.0, 1.0))
+        ball = torch.nn.functional.normalize(torch.randn((n, 3), generator=gen, device="cuda")) * 0.3
+        ball[:, 1] -= 0.7
+        return torch.where(torch.rand((n, 1), generator=gen, device="cuda") < 0.3, ball, p).contiguous()
+
+    pos, q = photons(1_000_000), photons(20_000)
+    one = torch.ones_like(pos)
+    ctx = photonmap.Context(0)
+    ctx.set_photons(0, pos, one, one)
+    ctx.build_grid(0, aabb=BOX)
+    qn = -q
+    near, far = (ctx.gather(q, qn, k, r, want_ids=True) for r in (0.5, 200.0))
+    for a, b in zip(near, far):
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+    assert bool((near[2] == k).all())
+    assert _time(ctx, q, qn, k, 200.0) < 2 * _time(ctx, q, qn, k, 0.5)
+    ctx.close()
