@@ -818,8 +818,8 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
             if (mode == M_WIDE || lim2 * m2 < s.block2) break;
             mode = M_WIDE;            // ... in the 27 sub-cells: with the guess that they give, or r
             lim2 = 9.f * E.sc * E.sc * GATHER_GUESS * __fdividef((float)k, 3.14159265f * (float)max(n, 1));
-        } else if (mode == M_WIDE) {  // the sphere held too few: a larger one
-            lim2 = lim2 * fmaxf(2.f, 1.5f * GATHER_GUESS * __fdividef((float)k, (float)max(n, 1)));
+        } else if (mode == M_WIDE) {  // the sphere held too few: a larger one, from the grid's diagonal on r's at once
+            lim2 = lim2 >= E.far2 ? E.r2 : lim2 * fmaxf(2.f, 1.5f * GATHER_GUESS * __fdividef((float)k, (float)max(n, 1)));
         } else {
             // the bound held too few of the 27: a larger one, then all of theirs, then
             // all within r.  (r at once: every photon of the 27 goes through the
@@ -1204,6 +1204,7 @@ GatherReach gather_reach(const GatherGrid& G, float r) {
     E.sc = G.cell / (float)G.S;
     E.inv_sc = 1.f / E.sc;
     E.ring2 = 12.5f * E.sc * E.sc;   // 3 (2 sc)^2 and a margin
+    E.far2 = G.cell * G.cell * ((float)G.gx * (float)G.gx + (float)G.gy * (float)G.gy + (float)G.gz * (float)G.gz);
     E.pad = G.cell * 1e-4f;
     return E;
 }

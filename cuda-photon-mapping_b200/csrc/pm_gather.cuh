@@ -33,6 +33,7 @@ struct GatherReach {
     float bscale;              // histogram bins / r2
     float sc, inv_sc;          // sub-cell edge, its reciprocal
     float ring2;               // squared distance within which the 27 sub-cells around a point of the grid lie
+    float far2;                // the grid's squared diagonal
     float pad;                 // boxes are taken this much larger
     int rc;                    // half width in cells of the reference's cube, ceil(r / cell)
                                // (CudaPhotonMapping/PhotonGrid.cu:257-284)

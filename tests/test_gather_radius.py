@@ -157,3 +157,25 @@ def test_time_does_not_grow_with_a_radius_that_holds_more_than_k(k):
     assert bool((near[2] == k).all())
     assert _time(ctx, q, qn, k, 200.0) < 2 * _time(ctx, q, qn, k, 0.5)
     ctx.close()
+
+
+@pytest.mark.gpu
+def test_time_does_not_grow_with_a_radius_beyond_few_photons():
+    """Fewer than k photons in a grid of many sub-cells: the walk ends soon after its
+    sphere has passed the grid, however large the radius."""
+    import torch
+    import photonmap
+    pos, power, inc = _map(255)
+    half = np.array([0.0625, 1, 1], np.float32)          # 1 x 16 x 16 cells, each cut 8 ways: 16,384 rows
+    pos *= half
+    q = torch.from_numpy(np.random.default_rng(3).uniform(-half, half, (500, 3)).astype(np.float32)).cuda()
+    ctx = photonmap.Context(0)
+    ctx.set_photons(0, pos, power, inc)
+    ctx.build_grid(0, aabb=np.concatenate([-half, half]), sub_div=8, desired=1)
+    assert ctx.photons(0)["dims"] == (1, 16, 16)
+    near, far = (ctx.gather(q, q, 256, r, want_ids=True) for r in (4.0, 1e18))
+    for a, b in zip(near, far):
+        assert torch.equal(a.view(torch.int32), b.view(torch.int32))
+    assert bool((near[2] == 255).all())
+    assert _time(ctx, q, q, 256, 1e18) < 3 * _time(ctx, q, q, 256, 4.0)
+    ctx.close()
