@@ -220,13 +220,14 @@ __global__ void k_key_count(const float* __restrict__ pos, int64_t n, GridGeom g
 }
 
 // key_starts of all sub-cells from the starts of those whose cell holds photons
-// (starts[rank * S^3 + sub-cell], the total last); cell_starts and cell_sizes.
+// (starts[rank * S^3 + sub-cell], the total last); cell_starts and cell_sizes
+// (which may be counts itself).
 // PER = 4 keys per thread (S > 1: of one cell), one 16-byte store; bound by the 4
 // bytes written per sub-cell (25.9M: 0.033 ms, one key per thread 0.099).
 template <int PER>
-__global__ void k_key_starts(const uint32_t* __restrict__ rank, const uint32_t* __restrict__ counts,
-                             const uint32_t* __restrict__ starts, int64_t keys, int sh, uint32_t* __restrict__ key_starts,
-                             uint32_t* __restrict__ cell_starts, uint32_t* __restrict__ cell_sizes) {
+__global__ void k_key_starts(const uint32_t* __restrict__ rank, const uint32_t* counts, const uint32_t* __restrict__ starts,
+                             int64_t keys, int sh, uint32_t* __restrict__ key_starts, uint32_t* __restrict__ cell_starts,
+                             uint32_t* cell_sizes) {
     const int64_t k = PER * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x);
     if (k >= keys) return;
     const int64_t c = k >> (3 * sh);
@@ -240,7 +241,7 @@ __global__ void k_key_starts(const uint32_t* __restrict__ rank, const uint32_t* 
     }
     if (s == 0u) {
         cell_starts[c] = from[0];
-        cell_sizes[c] = n;   // (may be counts itself)
+        if (cell_sizes != counts) cell_sizes[c] = n;
     }
     if (k + PER == keys) key_starts[keys] = from[n ? 1u << (3 * sh) : 0u];   // the total
 }

@@ -22,7 +22,7 @@ __device__ __forceinline__ unsigned long long poll(const unsigned long long* st)
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS)
-k_scan_u32(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int64_t n, int inclusive,
+k_scan_u32(const uint32_t* in, uint32_t* out, int64_t n, int inclusive,
            unsigned long long* tile_state, unsigned* tile_counter, uint32_t* total, unsigned* status,
            long long spin_limit, int silent_tile) {
     __shared__ uint32_t s_items[SCAN_TILE + SCAN_TILE / 32];

@@ -26,7 +26,8 @@ inline size_t scan_workspace_bytes(int64_t n) {
 }
 
 // exclusive (inclusive = 0) or inclusive scan of n u32 values; *total (device,
-// may be null) receives the sum of all n values.  ws: scan_workspace_bytes(n).
+// may be null) receives the sum of all n values.  out may be in (a tile reads its
+// values before it writes any).  ws: scan_workspace_bytes(n).
 // spin_limit: polls of one look-back wait before it gives up (ST_TIMEOUT);
 // silent_tile >= 0 (test hook only) makes that tile publish nothing, so every
 // later tile's look-back runs into the limit.
