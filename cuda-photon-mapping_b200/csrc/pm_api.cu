@@ -547,13 +547,14 @@ int pm_cache_gradient(pm_ctx* ctx, const float* pos, const float* nrm, const flo
         cudaGetLastError();
         ctx->hgrad = nullptr;
     }
-    if (int rc = cache_backprop(ctx, pos, nrm, target, weight, n, true, ctx->st)) return rc;
-    CK(cudaMemcpyAsync(ctx->hgrad ? ctx->hgrad : out_grad_host, ctx->cache_grad.p, (size_t)PM_CACHE_PARAMS * 4,
-                       cudaMemcpyDeviceToHost, ctx->st));
+    const bool paged = ctx->hgrad == nullptr;
+    if (int rc = cache_backprop(ctx, pos, nrm, target, weight, n, paged && out_loss, ctx->st)) return rc;
+    CK(cudaMemcpyAsync(paged ? out_grad_host : ctx->hgrad, ctx->cache_grad.p,
+                       (size_t)(PM_CACHE_PARAMS + (paged ? 0 : 1)) * 4, cudaMemcpyDeviceToHost, ctx->st));
     CK(cudaMemsetAsync(ctx->cache_grad.p, 0, (size_t)PM_CACHE_PARAMS * 4, ctx->st));
     const int rc = check_status(ctx, "cache gradient");
-    if (ctx->hgrad) std::memcpy(out_grad_host, ctx->hgrad, (size_t)PM_CACHE_PARAMS * 4);
-    if (out_loss) *out_loss = cache_loss_of(ctx, n);
+    if (!paged) std::memcpy(out_grad_host, ctx->hgrad, (size_t)PM_CACHE_PARAMS * 4);
+    if (out_loss) *out_loss = paged ? cache_loss_of(ctx, n) : ctx->hgrad[PM_CACHE_PARAMS] / (3.f * (float)n);
     return rc;
 }
 
