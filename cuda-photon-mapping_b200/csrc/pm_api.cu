@@ -205,12 +205,13 @@ int render_checks(pm_ctx* ctx, const pm_camera* cam, const pm_render_opts* o) {
 namespace {
 // the columns [c0, c1] and rows [r0, r1] that cover the pixels [i0, i1) of eye_pixel's order
 void eye_block_rect(int64_t i0, int64_t i1, int W, int H, int& c0, int& c1, int& r0, int& r1) {
-    const int64_t band = 4 * (int64_t)W;
-    r0 = (int)(i0 / band) * 4;
-    r1 = std::min((int)((i1 - 1) / band) * 4 + 3, H - 1);
+    const int64_t band = 4 * (int64_t)W, first = i0 / band;
+    const int64_t a = i0 - first * band, z = a + (i1 - i0);
+    r0 = (int)first * 4;
+    r1 = std::min((int)(z <= band ? first : (i1 - 1) / band) * 4 + 3, H - 1);
     c0 = 0;
     c1 = W - 1;
-    const int64_t a = i0 % band, z = a + (i1 - i0);   // one band's whole tiles: their columns
+    // one band's whole tiles: their columns
     if (r0 + 3 == r1 && z <= 4 * (int64_t)(W & ~31)) {
         c0 = (int)(a >> 7) * 32;
         c1 = (int)((z - 1) >> 7) * 32 + 31;
@@ -1323,14 +1324,13 @@ int render_eye_launch(pm_ctx* ctx, const pm_camera* cam, const pm_render_opts* o
     const int* order = P<int>(ctx->eye_order);
     int64_t nblocks = -1;
     if (y0 < y1) {
-        // the band's blocks, in the full order's (slow blocks first)
-        const int64_t T = eye_threads();
+        // the blocks with pixels in the bands of 4 rows that hold rows y0 .. y1 - 1, in
+        // the full order's (slow blocks first)
+        const int64_t T = eye_threads(), rows4 = 4 * (int64_t)cam->width;
+        const int64_t lo = y0 / 4 * rows4, hi = (y1 + 3) / 4 * rows4;
         std::vector<int> band;
-        for (int b : ctx->h_eye_order) {
-            int c0, c1, r0, r1;
-            eye_block_rect(b * T, std::min(b * T + T, F.npx), cam->width, cam->height, c0, c1, r0, r1);
-            if (r0 < y1 && r1 >= y0) band.push_back(b);
-        }
+        for (int b : ctx->h_eye_order)
+            if ((int64_t)b * T < hi && ((int64_t)b + 1) * T > lo) band.push_back(b);
         ENSURE(ctx->eye_band, std::max<size_t>(band.size(), 1) * 4);
         if (!band.empty())
             CK(cudaMemcpyAsync(ctx->eye_band.p, band.data(), band.size() * 4, cudaMemcpyHostToDevice, st));
