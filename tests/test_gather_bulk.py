@@ -30,8 +30,10 @@ def _bulk_equals_few(ctx, q, qn, n, k, radius):
     import torch
     m = q.shape[0]
     at = torch.arange(n, device="cuda") % m
+    many, many_n = q[at], qn[at]
+    torch.cuda.synchronize()                                   # the context has a stream of its own
     few = ctx.gather(q, qn, k, radius, want_ids=True)
-    bulk = ctx.gather(q[at], qn[at], k, radius, want_ids=True)
+    bulk = ctx.gather(many, many_n, k, radius, want_ids=True)
     for a, b in zip(few, bulk):
         # bits: a photon at its query alone gives 0 / 0
         a, b = (x.reshape(-1, x.numel() // r).view(torch.int32) for x, r in ((a, m), (b, n)))

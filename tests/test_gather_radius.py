@@ -147,10 +147,12 @@ def test_time_does_not_grow_with_a_radius_that_holds_more_than_k(k):
 
     pos, q = photons(1_000_000), photons(20_000)
     one = torch.ones_like(pos)
+    torch.cuda.synchronize()                             # the context has a stream of its own
     ctx = photonmap.Context(0)
     ctx.set_photons(0, pos, one, one)
     ctx.build_grid(0, aabb=BOX)
     qn = -q
+    torch.cuda.synchronize()
     near, far = (ctx.gather(q, qn, k, r, want_ids=True) for r in (0.5, 200.0))
     for a, b in zip(near, far):
         assert torch.equal(a.view(torch.int32), b.view(torch.int32))

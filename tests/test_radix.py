@@ -57,6 +57,7 @@ def test_running_counts_pass_from_lane_to_lane(n, m):
     pos = torch.zeros((n, 3), device="cuda")
     pos[:, 0] = (key.float() + 0.5) / 64
     pw = torch.full_like(pos, 0.5)
+    torch.cuda.synchronize()                                # the context has a stream of its own
     ctx = photonmap.Context(0)
     ctx.set_photons(0, pos, pw, pw)
     ctx.build_grid(0, aabb=BOX, sub_div=8, desired=-(-n // 512), regrid_mult=1000)   # 64 sub-cells along x
