@@ -445,8 +445,18 @@ __device__ __forceinline__ void stage_query(const GatherGrid& G, const GatherRea
                           face(q.z, G.mn[2], Z0, lz, hz)) - E.pad;
     const float block2 = f > 0.f ? f * f : 0.f;
     s.block2 = block2;
-    s.lim2 = N >= (uint32_t)k ? fminf(r2, tie_bound(E.ring2)) : r2;
-    if (G.guess > 0.f && N > (uint32_t)k) {   // else too few photons in the block to gain anything
+    // A query outside the grid (its sub-cell is then the nearest one): spheres are
+    // taken that much larger, and the guess says nothing.
+    auto beyond = [&](float p, float mn, int g) { return fmax3(mn - p, p - (mn + (float)g * G.cell), 0.f); };
+    const float ox = beyond(q.x, G.mn[0], G.gx), oy = beyond(q.y, G.mn[1], G.gy), oz = beyond(q.z, G.mn[2], G.gz);
+    const float out2 = ox * ox + oy * oy + oz * oz;
+    const bool outside = out2 > 0.25f * sc * sc;
+    auto bound = [&](float x) {
+        const float t = sqrt_approx(out2) + sqrt_approx(x);
+        return fminf(r2, tie_bound(outside ? t * t : x));
+    };
+    s.lim2 = N >= (uint32_t)k ? bound(outside ? 27.f * sc * sc : E.ring2) : r2;
+    if (G.guess > 0.f && N > (uint32_t)k && !outside) {   // else too few photons in the block to gain anything
         const float g2 = tie_bound(9.f * sc * sc * (G.guess * (float)k) / (3.14159265f * (float)N));
         if (g2 < r2) {
             s.lim2 = g2;
@@ -454,14 +464,16 @@ __device__ __forceinline__ void stage_query(const GatherGrid& G, const GatherRea
         }
     } else if (N < (uint32_t)k && !(r2 * BLOCK_MARGIN < block2)) {
         // fewer than k in the block and more of r's sphere beyond it: the
-        // sphere of the guess (at once that of r where it hardly leaves the
-        // block).  Where none of r's sphere lies beyond, the 27 sub-cells in the
+        // sphere of the guess, of at most eight sub-cells (a larger one that reaches
+        // a dense place meets its photons far side first, and the store overflows
+        // dozens of times), at once that of r where it hardly leaves the
+        // block.  Where none of r's sphere lies beyond, the 27 sub-cells in the
         // walk's own order, bound r, answer the query: as a growing sphere, its
         // answer ordered afterwards, 61,779 requests of the small room (k 100)
         // took 0.174 ms instead of 0.143.
         const float per = G.guess > 0.f ? G.guess : GATHER_GUESS;
         if (r2 > 4.f * sc * sc)
-            s.lim2 = fminf(r2, tie_bound(N > 0u ? 9.f * sc * sc * (per * (float)k) / (3.14159265f * (float)N) : 64.f * sc * sc));
+            s.lim2 = bound(fminf(9.f * sc * sc * (per * (float)k) / (3.14159265f * (float)N), 64.f * sc * sc));
         flags |= Q_WIDE;
     }
     s.qx = q.x; s.qy = q.y; s.qz = q.z;
@@ -664,7 +676,7 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
     float lim2 = s.lim2;       // a candidate enters when its squared distance <= lim2 (<= E.r2)
     float bscale = s.bscale;   // histogram bin of d2 = min(NB - 1, (int)(d2 * bscale))
     uint32_t found = 0u;       // find_bin's answer for a store of `fn`
-    int fn = -1;
+    int fn = -1;               // (-1: none; -2: none, and a larger bound was tried in the 27)
     int mode = s.flags & Q_WIDE ? M_WIDE : M_RING, base = 0, total = 27;
     bool coarse = false;       // M_WIDE: rows of cells, not of sub-cells
     bool plan = mode == M_WIDE;   // the box of rows is still to be set
@@ -822,7 +834,7 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
                 if (n > UCAP - 32) {
                     lim2 = fminf(lim2, overflow<UCAP>(U, G.gpos, n, k, bscale, lane));
                     n = U.box[7];
-                    fn = -1;
+                    fn = min(fn, -1);
                 }
             };
             int before = -1;
@@ -857,24 +869,28 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
         }
         if (lim2 == E.r2) {           // all within r is found ...
             if (mode == M_WIDE || lim2 * m2 < s.block2) break;
-            mode = M_WIDE;            // ... in the 27 sub-cells: with the guess that they give, or r
-            lim2 = 9.f * E.sc * E.sc * GATHER_GUESS * __fdividef((float)k, 3.14159265f * (float)max(n, 1));
+            mode = M_WIDE;            // ... in the 27 sub-cells, which hold k: r hardly leaves them
         } else if (mode == M_WIDE) {  // the sphere held too few: a larger one, from the grid's diagonal on r's at once
-            lim2 = lim2 >= E.far2 ? E.r2 : lim2 * fmaxf(2.f, 1.5f * GATHER_GUESS * __fdividef((float)k, (float)max(n, 1)));
+            lim2 = lim2 >= E.far2 ? E.r2 :
+                   lim2 * fminf(4.f, fmaxf(2.f, 1.5f * GATHER_GUESS * __fdividef((float)k, (float)max(n, 1))));
         } else {
-            // the bound held too few of the 27: a larger one, then all of theirs, then
-            // all within r.  (r at once: every photon of the 27 goes through the
-            // store, and the histogram over [0, r2] bounds nothing where r spans
-            // many sub-cells.  1,021 queries at k 16 62 -> 52 us, 100,003 at k 200
-            // 1.77 -> 1.60 ms; at a radius of 100 boxes 2.2 ms for 20,000, now 0.2.)
-            lim2 = lim2 < 0.99f * E.ring2 ? fminf(E.ring2, lim2 * GATHER_GUESS * __fdividef((float)k, (float)max(n, 1))) : E.r2;
+            // The bound held too few of the 27: once a larger one, unless so few that
+            // the guess says nothing here, then all of theirs, then all within r.  (r at
+            // once: every photon of the 27 goes through the store, and the histogram
+            // over [0, r2] bounds nothing where r spans many sub-cells.  1,021
+            // queries at k 16 62 -> 51 us, 100,003 at k 200 1.77 -> 1.60 ms; at a radius
+            // of 100 boxes 2.2 ms for 20,000, now 0.2.  Larger ones until one holds: each scans a
+            // dense sub-cell again, 273 queries at k 8 0.6 -> 1.2 ms.)
+            lim2 = lim2 >= 0.99f * E.ring2 ? E.r2 :
+                   fn == -2 || 4 * n + 4 < k ? E.ring2 :
+                   fminf(E.ring2, lim2 * __fdividef(GATHER_GUESS * (float)k + 4.f, (float)max(n, 1)));
+            fn = -2;
             plan = false;
         }
         lim2 = lim2 < E.r2 ? fminf(E.r2, tie_bound(lim2)) : E.r2;
         coarse = plan && lim2 > 16.f * E.sc * E.sc && E.sh > 0;
         bscale = lim2 == E.r2 ? E.bscale : __fdividef((float)NB, lim2);
         n = 0;
-        fn = -1;
         base = 0;
         reinterpret_cast<uint2*>(U.dh)[lane] = make_uint2(0u, 0u);
         __syncwarp();
