@@ -28,12 +28,13 @@
 // (z, y, x) order if those 27 hold k photons within r, else by shells of equal
 // Chebyshev distance (shell_index).
 //
-// What bounds it: instruction issue (0.76 of the issue slots; candidates come
-// from L1 / L2).  Against a store of 64-bit (distance, id) keys with a root per
-// candidate, sub-cells tested one by one and the set-up by the whole warp: 2,340 ->
-// 1,330 warp instructions per query and 3.03 -> 1.92 ms for the 1.23M queries
-// (k 64) of the 10M-photon 1080p frame; k 128 on 2M photons 2.12 -> 1.27 ms,
-// k 200 on 30M photons 7.0 -> 5.4 ms, k 32 on 500K photons 2.03 -> 1.27 ms.
+// What bounds it: instructions and the latency of the reads that each round of
+// 32 photons waits for (from L1 / L2): 1,417 warp instructions a query at 0.56 of
+// the issue slots for the 137K requests (k 64) of a 640 x 360 frame of 4M photons.
+// Against a store of 64-bit (distance, id) keys with a root per candidate, sub-cells
+// tested one by one and the set-up by the whole warp (2,233 at 0.70 there): 3.03 -> 1.92 ms for the 1.23M queries (k 64) of the 10M-photon 1080p frame; k 128
+// on 2M photons 2.12 -> 1.27 ms, k 200 on 30M photons 7.0 -> 5.4 ms, k 32 on 500K
+// photons 2.03 -> 1.27 ms.
 // Loops are not unrolled and the scan is there once: with three unrolled copies
 // the kernel waited for its instructions (2.6 of 10 stall cycles per issue,
 // 2.78 ms).  A dense caustic (60,000 photons in 27 sub-cells) makes single
@@ -179,6 +180,11 @@ __device__ __forceinline__ uint32_t nth_of_lanes(uint32_t mine, int got, uint32_
     return __shfl_sync(0xffffffffu, mine, __ffs(hit) - 1);
 }
 
+// (out of line: resolve_ties is called where registers are short)
+__device__ __noinline__ uint32_t nth_tie(const uint32_t* sel, int ties, uint32_t need, int lane) {
+    return nth_of_lanes(lane < ties ? sel[lane] : 0xffffffffu, ties, need, lane);
+}
+
 // Of w kept candidates more than k remain: some lie so close behind the
 // k-th squared distance that their rounded distances may tie with its own.
 // Order is (distance, source index): drop the largest.  Rare.
@@ -199,7 +205,7 @@ __device__ __noinline__ int resolve_ties(uint2* ent, uint32_t* sel, const float4
     const int need = k - below;   // ties that stay, smallest source index first
     uint32_t id_max = 0xffffffffu;
     if (ties > need && ties <= 32) {
-        id_max = nth_of_lanes(lane < ties ? sel[lane] : 0xffffffffu, ties, (uint32_t)need, lane);
+        id_max = nth_tie(sel, ties, (uint32_t)need, lane);
     } else if (ties > need) {
         id_max = 0u;              // the need-th smallest index among the ties
 #pragma unroll 1
@@ -480,6 +486,26 @@ __device__ __forceinline__ void stage_query(const GatherGrid& G, const GatherRea
     s.X0 = X0; s.Y0 = Y0; s.Z0 = Z0;
     s.flags = flags;
     s.bscale = (float)NB / s.lim2;
+}
+
+// The bound with which a walk goes on that found n < k photons within lim2 (below r2).
+// A sphere (wide): a larger one, from the grid's diagonal on r's at once.  The 27
+// sub-cells: once a larger bound, unless so few were found that the count says
+// nothing here, then all of theirs, then all within r.  (r at once: every photon of
+// the 27 goes through the store, and the histogram over [0, r2] bounds nothing where r
+// spans many sub-cells.  1,021 queries at k 16 62 -> 51 us, 100,003 at k 200
+// 1.77 -> 1.60 ms; at a radius of 100 boxes 2.2 ms for 20,000, now 0.2.  Larger ones
+// until one holds: each scans a dense sub-cell again, 273 queries at k 8 0.6 -> 1.2 ms.)
+// Out of line, as the other rare parts are: the walk then takes fewer registers
+// and instruction lines (30M photons, k 200: 5.57 -> 5.41 ms).
+__device__ __noinline__ float next_bound(float lim2, int n, int k, bool wide, bool once, float r2, float ring2, float far2) {
+    const float per = __fdividef(1.f, (float)max(n, 1));
+    float x;
+    if (wide) x = lim2 >= far2 ? r2 : lim2 * fminf(4.f, fmaxf(2.f, 1.5f * GATHER_GUESS * (float)k * per));
+    else if (lim2 >= 0.99f * ring2) x = r2;
+    else if (once || 4 * n + 4 < k) x = ring2;
+    else x = fminf(ring2, lim2 * (GATHER_GUESS * (float)k + 4.f) * per);
+    return x < r2 ? fminf(r2, tie_bound(x)) : r2;
 }
 
 // Sub-cells [range_low, range_high] along an axis hold every photon within
@@ -870,26 +896,13 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
         if (lim2 == E.r2) {           // all within r is found ...
             if (mode == M_WIDE || lim2 * m2 < s.block2) break;
             mode = M_WIDE;            // ... in the 27 sub-cells, which hold k: r hardly leaves them
-        } else if (mode == M_WIDE) {  // the sphere held too few: a larger one, from the grid's diagonal on r's at once
-            lim2 = lim2 >= E.far2 ? E.r2 :
-                   lim2 * fminf(4.f, fmaxf(2.f, 1.5f * GATHER_GUESS * __fdividef((float)k, (float)max(n, 1))));
         } else {
-            // The bound held too few of the 27: once a larger one, unless so few that
-            // the guess says nothing here, then all of theirs, then all within r.  (r at
-            // once: every photon of the 27 goes through the store, and the histogram
-            // over [0, r2] bounds nothing where r spans many sub-cells.  1,021
-            // queries at k 16 62 -> 51 us, 100,003 at k 200 1.77 -> 1.60 ms; at a radius
-            // of 100 boxes 2.2 ms for 20,000, now 0.2.  Larger ones until one holds: each scans a
-            // dense sub-cell again, 273 queries at k 8 0.6 -> 1.2 ms.)
-            lim2 = lim2 >= 0.99f * E.ring2 ? E.r2 :
-                   fn == -2 || 4 * n + 4 < k ? E.ring2 :
-                   fminf(E.ring2, lim2 * __fdividef(GATHER_GUESS * (float)k + 4.f, (float)max(n, 1)));
+            lim2 = next_bound(lim2, n, k, mode == M_WIDE, fn == -2, E.r2, E.ring2, E.far2);
+            plan = mode == M_WIDE;
             fn = -2;
-            plan = false;
         }
-        lim2 = lim2 < E.r2 ? fminf(E.r2, tie_bound(lim2)) : E.r2;
         coarse = plan && lim2 > 16.f * E.sc * E.sc && E.sh > 0;
-        bscale = lim2 == E.r2 ? E.bscale : __fdividef((float)NB, lim2);
+        bscale = __fdividef((float)NB, lim2);
         n = 0;
         base = 0;
         reinterpret_cast<uint2*>(U.dh)[lane] = make_uint2(0u, 0u);
@@ -1251,7 +1264,6 @@ GatherReach gather_reach(const GatherGrid& G, float r) {
         while (s < FLT_MAX && std::sqrt(std::nextafter(s, INFINITY)) <= r) s = std::nextafter(s, INFINITY);
         E.r2 = s;
     }
-    E.bscale = (float)NB / E.r2;
     const float c = std::ceil(r / G.cell);
     E.rc = c != c ? 0 : (int)std::min(std::max(c, -1e9f), 1e9f);
     E.sh = 0;

@@ -30,7 +30,6 @@ struct GatherReach {
     float r;
     float r2;                  // largest float s with sqrtf(s) <= r (-1 if none): a photon at squared
                                // distance s lies within r exactly when s <= r2
-    float bscale;              // histogram bins / r2
     float sc, inv_sc;          // sub-cell edge, its reciprocal
     float ring2;               // squared distance within which the 27 sub-cells around a point of the grid lie
     float far2;                // the grid's squared diagonal

@@ -12,7 +12,7 @@
 //                  resolution and the re-grid one) and their largest counts
 //                  (shared-memory counters + k_count_max when both grids fit)
 //                  -> host decides on the re-grid and on S
-//   k_cell_flags + scan_u32   rank of each cell among those that hold photons
+//   k_cell_rank (many cells: k_cell_flags + scan_u32)   rank of each cell among those that hold photons
 //   k_key_count    key = rank * S^3 + sub-cell per photon + key counts
 //   scan_u32       exclusive scan of key counts (decoupled look-back)
 //   k_key_starts   key_starts of all sub-cells; cell_starts, cell_sizes
