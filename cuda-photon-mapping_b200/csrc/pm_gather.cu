@@ -32,9 +32,10 @@
 // 32 photons waits for (from L1 / L2): 1,417 warp instructions a query at 0.56 of
 // the issue slots for the 137K requests (k 64) of a 640 x 360 frame of 4M photons.
 // Against a store of 64-bit (distance, id) keys with a root per candidate, sub-cells
-// tested one by one and the set-up by the whole warp (2,233 at 0.70 there): 3.03 -> 1.92 ms for the 1.23M queries (k 64) of the 10M-photon 1080p frame; k 128
-// on 2M photons 2.12 -> 1.27 ms, k 200 on 30M photons 7.0 -> 5.4 ms, k 32 on 500K
-// photons 2.03 -> 1.27 ms.
+// tested one by one and the set-up by the whole warp (2,233 at 0.70 there): 3.03 ->
+// 1.91 ms for the 1.23M queries (k 64) of the 10M-photon 1080p frame; k 128 on 2M
+// photons 2.12 -> 1.27 ms, k 200 on 30M photons 7.0 -> 5.4 ms, k 32 on 500K photons
+// 2.03 -> 1.27 ms.
 // Loops are not unrolled and the scan is there once: with three unrolled copies
 // the kernel waited for its instructions (2.6 of 10 stall cycles per issue,
 // 2.78 ms).  A dense caustic (60,000 photons in 27 sub-cells) makes single
@@ -64,7 +65,7 @@ struct WarpStore {
     uint32_t qa[QCAP];        // queued runs of consecutive slots: first slot, length
     uint32_t qc[QCAP];
     uint32_t sel[32];
-    int box[8];               // the box of rows being scanned: x0, x1, y0, rows along y, z0, runs per row, -, overflow's count
+    int box[8];               // the box of rows being scanned: x0, x1, y0, rows along y, z0, runs per row; [7]: overflow's count
 };
 
 // A query as the set-up (one thread per query) leaves it for its warp.
@@ -280,7 +281,8 @@ __device__ __forceinline__ uint32_t pick_s(WarpStore<UCAP>& U, int n, uint32_t l
 // the whole store it took up to 31 passes instead of about three: frame with a
 // caustic map 4.49 -> 4.29 ms, 2,027 queries at k 200 among clusters 1.99 -> 1.43.
 template <int UCAP>
-__device__ __noinline__ float kth_of_full_bin(WarpStore<UCAP>& U, int n, uint32_t need, uint32_t bin, float bscale, int lane) {
+__device__ __noinline__ float kth_of_full_bin(WarpStore<UCAP>& U, int n, uint32_t need, uint32_t bin, float bscale,
+                                              int lane) {
     uint32_t lo = 0xffffffffu, hi = 0u;
 #pragma unroll 1
     for (int i = lane; i < n; i += 32) {
@@ -873,7 +875,8 @@ __device__ __forceinline__ void gather_query(const GatherGrid& G, const GatherRe
                 const float4 p = __ldg(G.gpos + j);
                 const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
                 const float d2 = dx * dx + dy * dy + dz * dz;
-                enter(p0 + lane < photons ? d2 : __int_as_float(0x7fffffff), j);   // NaN is within no bound, infinity within that of r = inf
+                // (NaN: within no bound; infinity is within that of r = inf)
+                enter(p0 + lane < photons ? d2 : __int_as_float(0x7fffffff), j);
             }
         }
         qn = 0;
